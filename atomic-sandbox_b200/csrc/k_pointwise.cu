@@ -147,17 +147,25 @@ __global__ void lincomb_kernel(long long n4, float4* __restrict__ y, Terms t) {
     }
 }
 
-// out_j = sum_i C_ij S_i for up to QG outputs per CTA row (blockIdx.y picks the output group). The CTA
-// stages its slice of the m inputs (LCB float4 of each field, m x 2 KB: at most 128 KB for m = 64) in
-// shared memory with one cp.async.bulk per field, all completing on one mbarrier, so the whole slice is
-// in flight at once without holding registers; each thread then combines its float4 with packed f32x2
-// FMAs, in input order: the same roundings as one fmaf chain per output element.
-// m = 24, q = 16 at 95^3: the whole H2O solve 1.7 % faster than loading the inputs four at a time
-// through registers (bitwise-identical results). The FMA pairs are two OUTPUTS of one component,
-// (c_ij, c_ij+1) x (v_k, v_k), so one 16-byte shared load brings four coefficients: 5 shared loads per
-// input instead of 17 (coefficient pairs (c, c) per output), 37.6 instead of 47.3 us per launch.
-constexpr int QG = 16;
-constexpr int LCB = 128;  // float4 per field per CTA = threads per CTA
+// out_j = sum_i C_ij S_i: one persistent CTA per SM streams slices of the m inputs (LCB float4 of each field) through a
+// ring of shared-memory stages, each filled by one cp.async.bulk per field on the stage's mbarrier, so the next stages'
+// copies run behind the current ones' arithmetic and every input is read once whatever the number of outputs. A stage is
+// consumed by a set of LCB threads per group of QG outputs. The ring is a multiple of the sets, so a stage slot always
+// belongs to the same set, which therefore sees each of its barriers' phases (a set that skipped one could take the phase
+// before for its own). A thread combines its float4 of every input, in input order, with packed f32x2 FMAs whose pairs are
+// two OUTPUTS of one component, (c_ij, c_ij+1) x (v_k, v_k): one 16-byte shared load brings four coefficients, and the
+// roundings are those of one fmaf chain per output. The last group's missing outputs have zero coefficients and are
+// not stored: a test per output inside the loop kept its shared loads from being issued ahead. Bound by the shared loads
+// of the inputs (once per group of QG outputs) beside HBM. One CTA per slice and group of 16 outputs (the form this
+// replaces) read every input once per group from L2 and had no copy behind its arithmetic: m = 60, q = 40 on 128^3
+// 858 -> 253 us per launch (of 128 us for the bytes), m = 24, q = 16 on 95^3 37.0 -> 32.6 us. Two groups of 16 outputs
+// per thread measured slower (registers), 2 and 4 sets no faster than 3.
+constexpr int QG = 8;
+constexpr int LCB = 64;          // float4 per field per stage: 1 KB copies
+constexpr int LC_RING = 16;      // stages at most
+constexpr int LC_SETS = 3;
+constexpr int LC_THREADS = 960;  // consumer threads at most (with the producer warp 992: 64 registers each)
+constexpr int LC_SMEM = 216 * 1024;
 constexpr long long LC_WAIT_LIMIT = 1LL << 22;
 __device__ __forceinline__ unsigned long long lc_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
     unsigned long long d;
@@ -165,100 +173,129 @@ __device__ __forceinline__ unsigned long long lc_fma2(unsigned long long a, unsi
     return d;
 }
 __device__ __forceinline__ unsigned lc_su32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+// bounded wait: false when the barrier's phase did not complete within `limit` polls
+__device__ __forceinline__ bool lc_wait(uint64_t* bar, unsigned parity, long long limit) {
+    for (long long n = 0;; ++n) {
+        unsigned ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(lc_su32(bar)), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+        if (n > limit) return false;
+    }
+}
 
-__global__ void __launch_bounds__(LCB) block_lincomb_kernel(long long F4, int m, const ulonglong2* __restrict__ S, int q,
-                                                            const double* __restrict__ C, ulonglong2* __restrict__ out, int split,
-                                                            int gap, int* err) {
-    extern __shared__ __align__(128) ulonglong2 sv[];  // m x LCB
-    __shared__ __align__(16) float cs[64 * QG];        // c_ij at [i][jj], zero past the group's last output
-    __shared__ __align__(8) uint64_t bar;
-    const long long e0 = (long long)blockIdx.x * LCB;
-    const int cnt = (int)min((long long)LCB, F4 - e0);  // >= 1: the grid is ceil(F4 / LCB)
-    const unsigned bytes = (unsigned)cnt * 16u;          // a multiple of 16, from 16-byte aligned field rows
+struct LincombShape { int groups, sets, ring, slices; };
+
+__global__ void __launch_bounds__(LC_THREADS + 32, 1) block_lincomb_kernel(long long F4, int m, const ulonglong2* __restrict__ S, int q,
+                                                                           const double* __restrict__ C, ulonglong2* __restrict__ out,
+                                                                           int split, int gap, LincombShape sh, int* err) {
+    extern __shared__ __align__(128) ulonglong2 lc_buf[];  // ring x m x LCB, then the coefficients
+    __shared__ __align__(8) uint64_t full[LC_RING], empty[LC_RING];
+    const int set_threads = LCB * sh.groups, consumers = set_threads * sh.sets;
+    const int nmine = (sh.slices - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // slices blockIdx.x + k * gridDim.x
+    const int stage = m * LCB;
+    float* cs = reinterpret_cast<float*>(lc_buf + (size_t)sh.ring * stage);  // c_ij at [group][i][jj], zero past the last output
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(lc_su32(&bar)) : "memory");
+        for (int i = 0; i < sh.ring; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(lc_su32(&full[i])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(lc_su32(&empty[i])), "r"(set_threads / 32) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        if (threadIdx.x == 0)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(lc_su32(&bar)), "r"(bytes * (unsigned)m)
-                         : "memory");
-        __syncwarp();
-        for (int i = threadIdx.x; i < m; i += 32)
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                             lc_su32(sv + (size_t)i * LCB)),
-                         "l"(S + (long long)i * F4 + e0), "r"(bytes), "r"(lc_su32(&bar))
-                         : "memory");
-    }
-    // the coefficients while the copies are in flight
-    const int j0 = blockIdx.y * QG;
-    const int qn = min(QG, q - j0);
-    for (int t = threadIdx.x; t < m * QG; t += blockDim.x) {
-        const int i = t / QG, jj = t % QG;
-        cs[t] = jj < qn ? (float)C[i + (size_t)m * (j0 + jj)] : 0.0f;
-    }
-    __syncthreads();
-    // bounded wait on the copies: on timeout the error flag is raised (the host's next readback reports it) and the
-    // outputs are undefined; a second bounded wait then gives the copies in flight time to land before the CTA exits
-    // and its shared memory is reused
-    auto wait_copies = [&](long long limit) {
-        for (long long n = 0;; ++n) {
-            unsigned ok;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok)
-                         : "r"(lc_su32(&bar))
-                         : "memory");
-            if (ok) return true;
-            if (n > limit) return false;
+    if ((int)threadIdx.x >= consumers) {
+        // ---- producer warp. A wait that gives up raises the error flag (the host's next readback reports it) and ends the
+        // loads; the copies in flight then get a bounded time to land before the CTA's shared memory is released.
+        const int lane = threadIdx.x & 31;
+        int sl = 0, issued = 0;
+        unsigned ph = 1;  // a fresh barrier passes a wait on the parity before its first phase
+        bool alive = true;
+        for (; issued < nmine; ++issued) {
+            if (!lc_wait(&empty[sl], ph, LC_WAIT_LIMIT)) {
+                if (err) atomicExch(err, 1);
+                alive = false;
+                break;
+            }
+            // the consumers' reads of the slot come before the copies' writes, which are the async proxy's
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            const long long e0 = ((long long)blockIdx.x + (long long)issued * gridDim.x) * LCB;
+            const unsigned bytes = (unsigned)min((long long)LCB, F4 - e0) * 16u;  // a multiple of 16, from 16-byte aligned fields
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(lc_su32(&full[sl])), "r"(bytes * (unsigned)m)
+                             : "memory");
+            __syncwarp();
+            for (int i = lane; i < m; i += 32)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 lc_su32(lc_buf + (size_t)sl * stage + i * LCB)),
+                             "l"(S + (long long)i * F4 + e0), "r"(bytes), "r"(lc_su32(&full[sl]))
+                             : "memory");
+            if (++sl == sh.ring) { sl = 0; ph ^= 1u; }
         }
-    };
-    if (!wait_copies(LC_WAIT_LIMIT)) {
-        if (err) atomicExch(err, 1);
-        wait_copies(1LL << 16);
+        if (!__all_sync(0xffffffffu, alive))
+            for (int j = max(0, issued - sh.ring); j < issued; ++j) lc_wait(&full[j % sh.ring], (unsigned)((j / sh.ring) & 1), 1LL << 16);
+        return;
     }
-    const int tid = threadIdx.x;
-    if (tid >= cnt) return;
-    // acc[p][k]: component k of outputs (2p, 2p + 1)
-    unsigned long long acc[QG / 2][4];
+    // the coefficients while the first copies are in flight
+    for (int t = threadIdx.x; t < sh.groups * m * QG; t += consumers) {
+        const int jj = t % QG, i = (t / QG) % m, j = t / (QG * m) * QG + jj;
+        cs[t] = j < q ? (float)C[i + (size_t)m * j] : 0.0f;
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(consumers) : "memory");
+    const int set = threadIdx.x / set_threads, within = threadIdx.x % set_threads;
+    const int col = within % LCB, group = within / LCB;
+    const int j0 = group * QG, qn = min(QG, q - j0);
+    const ulonglong2* cs4 = reinterpret_cast<const ulonglong2*>(cs + (size_t)group * m * QG);
+    int sl = set;
+    unsigned ph = 0;
+    for (int k = set; k < nmine; k += sh.sets) {
+        if (!lc_wait(&full[sl], ph, LC_WAIT_LIMIT)) {
+            if (err) atomicExch(err, 1);
+            break;  // the outputs are undefined
+        }
+        const float4* sv = reinterpret_cast<const float4*>(lc_buf + (size_t)sl * stage) + col;
+        // acc[p][k]: component k of outputs (2p, 2p + 1)
+        unsigned long long acc[QG / 2][4];
 #pragma unroll
-    for (int p = 0; p < QG / 2; ++p) acc[p][0] = acc[p][1] = acc[p][2] = acc[p][3] = 0ull;
-    const float4* sv4 = reinterpret_cast<const float4*>(sv);
-    const ulonglong2* cs4 = reinterpret_cast<const ulonglong2*>(cs);
+        for (int p = 0; p < QG / 2; ++p) acc[p][0] = acc[p][1] = acc[p][2] = acc[p][3] = 0ull;
 #pragma unroll 4
-    for (int i = 0; i < m; ++i) {
-        const float4 v = sv4[(size_t)i * LCB + tid];
-        unsigned long long vv[4];  // (v.k, v.k)
-        asm("mov.b64 %0, {%1, %1};" : "=l"(vv[0]) : "f"(v.x));
-        asm("mov.b64 %0, {%1, %1};" : "=l"(vv[1]) : "f"(v.y));
-        asm("mov.b64 %0, {%1, %1};" : "=l"(vv[2]) : "f"(v.z));
-        asm("mov.b64 %0, {%1, %1};" : "=l"(vv[3]) : "f"(v.w));
+        for (int i = 0; i < m; ++i) {
+            const float4 v = sv[i * LCB];
+            unsigned long long vv[4];  // (v.k, v.k)
+            asm("mov.b64 %0, {%1, %1};" : "=l"(vv[0]) : "f"(v.x));
+            asm("mov.b64 %0, {%1, %1};" : "=l"(vv[1]) : "f"(v.y));
+            asm("mov.b64 %0, {%1, %1};" : "=l"(vv[2]) : "f"(v.z));
+            asm("mov.b64 %0, {%1, %1};" : "=l"(vv[3]) : "f"(v.w));
 #pragma unroll
-        for (int p4 = 0; p4 < QG / 4; ++p4) {
-            if (4 * p4 < qn) {
+            for (int p4 = 0; p4 < QG / 4; ++p4) {
                 const ulonglong2 c4 = cs4[i * (QG / 4) + p4];  // (c_4p4, c_4p4+1), (c_4p4+2, c_4p4+3)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) acc[2 * p4][k] = lc_fma2(c4.x, vv[k], acc[2 * p4][k]);
-                if (4 * p4 + 2 < qn) {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) acc[2 * p4 + 1][k] = lc_fma2(c4.y, vv[k], acc[2 * p4 + 1][k]);
+                for (int k2 = 0; k2 < 4; ++k2) {
+                    acc[2 * p4][k2] = lc_fma2(c4.x, vv[k2], acc[2 * p4][k2]);
+                    acc[2 * p4 + 1][k2] = lc_fma2(c4.y, vv[k2], acc[2 * p4 + 1][k2]);
                 }
             }
         }
-    }
-    const long long e = e0 + tid;
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(lc_su32(&empty[sl])) : "memory");
+        sl += sh.sets;
+        if (sl >= sh.ring) { sl -= sh.ring; ph ^= 1u; }
+        const long long e = ((long long)blockIdx.x + (long long)k * gridDim.x) * LCB + col;
+        if (e >= F4) continue;
 #pragma unroll
-    for (int p = 0; p < QG / 2; ++p) {
-        unsigned lo[4], hi[4];
+        for (int p = 0; p < QG / 2; ++p) {
+            unsigned lo[4], hi[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) asm("mov.b64 {%0, %1}, %2;" : "=r"(lo[k]), "=r"(hi[k]) : "l"(acc[p][k]));
-        const int ja = j0 + 2 * p, jb = ja + 1;
-        if (2 * p < qn)
-            out[(long long)(ja < split ? ja : ja + gap) * F4 + e] =
-                make_ulonglong2(lo[0] | ((unsigned long long)lo[1] << 32), lo[2] | ((unsigned long long)lo[3] << 32));
-        if (2 * p + 1 < qn)
-            out[(long long)(jb < split ? jb : jb + gap) * F4 + e] =
-                make_ulonglong2(hi[0] | ((unsigned long long)hi[1] << 32), hi[2] | ((unsigned long long)hi[3] << 32));
+            for (int k2 = 0; k2 < 4; ++k2) asm("mov.b64 {%0, %1}, %2;" : "=r"(lo[k2]), "=r"(hi[k2]) : "l"(acc[p][k2]));
+            const int ja = j0 + 2 * p, jb = ja + 1;
+            if (2 * p < qn)
+                out[(long long)(ja < split ? ja : ja + gap) * F4 + e] =
+                    make_ulonglong2(lo[0] | ((unsigned long long)lo[1] << 32), lo[2] | ((unsigned long long)lo[3] << 32));
+            if (2 * p + 1 < qn)
+                out[(long long)(jb < split ? jb : jb + gap) * F4 + e] =
+                    make_ulonglong2(hi[0] | ((unsigned long long)hi[1] << 32), hi[2] | ((unsigned long long)hi[3] << 32));
+        }
     }
 }
 
@@ -494,14 +531,20 @@ void launch_block_lincomb(long long F, int m, const float* S, int q, const doubl
     // the bulk copies need 16-byte aligned sources and sizes: whole float4 rows of 16-byte aligned fields
     if (F % 4 != 0 || reinterpret_cast<uintptr_t>(S) % 16 != 0 || reinterpret_cast<uintptr_t>(out) % 16 != 0)
         throw std::invalid_argument("block_lincomb: fields must be 16-byte aligned with F a multiple of 4 floats");
-    long long F4 = F / 4;
+    const long long F4 = F / 4;
     static std::atomic<unsigned long long> attr_set{0};
-    once_per_device(attr_set, [] {  // 64 fields x LCB float4 of dynamic shared memory at most
-        KS_CUDA(cudaFuncSetAttribute(block_lincomb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * LCB * 16));
-    });
-    dim3 grid((unsigned)((F4 + LCB - 1) / LCB), ceil_div(q, QG));
-    block_lincomb_kernel<<<grid, LCB, (size_t)m * LCB * 16, s>>>(F4, m, reinterpret_cast<const ulonglong2*>(S), q, C,
-                                                                 reinterpret_cast<ulonglong2*>(out), split, gap, device_error_flag());
+    once_per_device(attr_set, [] { KS_CUDA(cudaFuncSetAttribute(block_lincomb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LC_SMEM)); });
+    LincombShape sh;
+    sh.groups = ceil_div(q, QG);
+    if (sh.groups * LCB > LC_THREADS) throw std::invalid_argument("block_lincomb: at most 120 outputs");
+    const int stage_bytes = m * LCB * 16, coef_bytes = sh.groups * m * QG * 4;
+    sh.ring = std::min(LC_RING, (LC_SMEM - coef_bytes) / stage_bytes);  // >= 2 (m = 64: 64 KB)
+    sh.sets = std::min(LC_THREADS / (sh.groups * LCB), std::min(LC_SETS, sh.ring));
+    sh.ring -= sh.ring % sh.sets;
+    sh.slices = (int)((F4 + LCB - 1) / LCB);
+    const int grid = std::min(sm_count(), sh.slices);
+    block_lincomb_kernel<<<grid, sh.sets * sh.groups * LCB + 32, sh.ring * stage_bytes + coef_bytes, s>>>(
+        F4, m, reinterpret_cast<const ulonglong2*>(S), q, C, reinterpret_cast<ulonglong2*>(out), split, gap, sh, device_error_flag());
     KS_LAUNCH_CHECK();
 }
 
