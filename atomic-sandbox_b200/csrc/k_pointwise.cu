@@ -218,8 +218,6 @@ __global__ void __launch_bounds__(LC_THREADS + 32, 1) block_lincomb_kernel(long 
                 alive = false;
                 break;
             }
-            // the consumers' reads of the slot come before the copies' writes, which are the async proxy's
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             const long long e0 = ((long long)blockIdx.x + (long long)issued * gridDim.x) * LCB;
             const unsigned bytes = (unsigned)min((long long)LCB, F4 - e0) * 16u;  // a multiple of 16, from 16-byte aligned fields
             if (lane == 0)
@@ -277,6 +275,8 @@ __global__ void __launch_bounds__(LC_THREADS + 32, 1) block_lincomb_kernel(long 
                 }
             }
         }
+        // these reads of the slot come before the writes of the copies that refill it, which are the async proxy's
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(lc_su32(&empty[sl])) : "memory");
         sl += sh.sets;
