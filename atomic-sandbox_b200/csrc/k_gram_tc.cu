@@ -119,10 +119,7 @@ __device__ __forceinline__ float tf32_rn(float x) { return __uint_as_float((__fl
 struct Params {
     long long F;  // points per field (multiple of 4)
     int m, mt;
-    int P;        // 32-point slabs per stage (2 when m and mt fit 32-row blocks, else 1)
-    int SB;       // row stride of the S blocks of a stage's slabs
-    int TR0, TB;  // first T row, row stride of the T blocks
-    int N;        // MMA N: rows of the tile used as the B operand
+    int TR0;      // first T row = MMA N: rows of the tile used as the B operand
     int rows;     // rows the split converts
     int stages_total;
     int R;        // ring depth
@@ -144,8 +141,8 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
     __shared__ unsigned tmem_base;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nbuf = min(NBUF_MAX, 512 / (2 * p.N));  // TMEM: nbuf buffers of two N-column slots (hi*hi, cross)
-    // this CTA's contiguous range of stages (P slabs of 32 points each)
+    const int nbuf = min(NBUF_MAX, 512 / (2 * p.TR0));  // TMEM: nbuf buffers of two N-column slots (hi*hi, cross)
+    // this CTA's contiguous range of stages (32 points each)
     const int per = (p.stages_total + gridDim.x - 1) / gridDim.x;
     const int s0 = blockIdx.x * per;
     const int s1 = min(p.stages_total, s0 + per);
@@ -177,20 +174,18 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
     const unsigned tmem = tmem_base;
 
     if (warp == 12) {
-        // ---- TMA producer: slab q of a stage puts its S rows at row q*SB, its T rows at TR0 + q*TB
+        // ---- TMA producer: a stage's S rows at row 0, its T rows at TR0
         if (lane == 0) {
-            const unsigned bytes = (unsigned)(p.P * (p.m + p.mt) * KT * 4);
+            const unsigned bytes = (unsigned)((p.m + p.mt) * KT * 4);
             int s = 0;
             unsigned ph = 0;
             for (int i = 0; i < nst; ++i) {
                 if (i >= R && !mbar_wait(&empty[s], ph ^ 1u, p.err)) break;
                 mbar_expect_tx(&full[s], bytes);
                 unsigned char* dst = hi + (size_t)s * p.tbytes;
-                for (int q = 0; q < p.P; ++q) {
-                    const int x = ((s0 + i) * p.P + q) * KT;
-                    tma_2d(dst + q * p.SB * KT * 4, &tm_s, x, 0, &full[s]);
-                    tma_2d(dst + (p.TR0 + q * p.TB) * KT * 4, &tm_t, x, 0, &full[s]);
-                }
+                const int x = (s0 + i) * KT;
+                tma_2d(dst, &tm_s, x, 0, &full[s]);
+                tma_2d(dst + p.TR0 * KT * 4, &tm_t, x, 0, &full[s]);
                 if (++s == R) { s = 0; ph ^= 1u; }
             }
         }
@@ -232,7 +227,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
         // whole-range cross-term slot biased the Gram by ~1e-7 relative). Descriptors advance by the
         // tile size (ring) and 32 B per K-step (the address field counts 16-byte units).
         if (lane == 0) {
-            const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(p.N >> 3) << 17) | ((unsigned)(ROWS >> 4) << 24);
+            const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(p.TR0 >> 3) << 17) | ((unsigned)(ROWS >> 4) << 24);
             const unsigned long long dh0 = smem_desc(su32(hi)), dl0 = smem_desc(su32(lo));
             const unsigned long long step = (unsigned long long)(p.tbytes >> 4);
             const bool main_issuer = warp == 13;
@@ -242,7 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
                 if (i >= nbuf && !mbar_wait(&acc_empty[b], bph ^ 1u, p.err)) break;
                 if (!mbar_wait(&conv[s], ph, p.err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned d = tmem + (unsigned)(2 * b * p.N) + (main_issuer ? 0u : (unsigned)p.N);
+                const unsigned d = tmem + (unsigned)(2 * b * p.TR0) + (main_issuer ? 0u : (unsigned)p.TR0);
                 const unsigned long long h0 = dh0 + (unsigned long long)s * step, l0 = dl0 + (unsigned long long)s * step;
                 if (main_issuer) {
                     mma_tf32(d, h0, h0, idesc, 0u);
@@ -267,34 +262,24 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
         // ---- epilogue: warps 0..7; warp w reads TMEM lanes 32(w%4)..+31 (row = lane index) and the
         // column half w/4 of its rows' own N-column block. Each stage's two slots (hi*hi and cross
         // terms) are added to f32 sums (round-to-nearest), which go into f64 totals every FLUSH
-        // stages. With two slabs per stage, lane quadrants 0..3 hold S of slab 0, S of slab 1,
-        // T of slab 0, T of slab 1, and slab q's columns start at 32q.
+        // stages.
         constexpr int HALF = NMAX / 2;
         const int quad = warp & 3, c0 = (warp >> 2) * HALF;
         const int mc = (p.m + 7) & ~7;  // columns of D that hold data
-        int orow, colbase, slab;
-        if (p.P == 2) {
-            slab = quad & 1;
-            colbase = 32 * slab;
-            orow = (quad < 2) ? (lane < p.m ? lane : -1) : (lane < p.mt ? p.m + lane : -1);
-        } else {
-            const int r = quad * 32 + lane;
-            slab = 0;
-            colbase = 0;
-            orow = r < p.m ? r : (r >= p.TR0 && r < p.TR0 + p.mt ? r - p.TR0 + p.m : -1);
-        }
+        const int r = quad * 32 + lane;
+        const int orow = r < p.m ? r : (r >= p.TR0 && r < p.TR0 + p.mt ? r - p.TR0 + p.m : -1);
         const int ncols = max(0, min(HALF, mc - c0));  // multiple of 8, the same for the whole warp
         float fs[HALF];
         double acc[HALF];
 #pragma unroll
         for (int j = 0; j < HALF; ++j) { fs[j] = 0.f; acc[j] = 0.0; }
-        const unsigned lane_base = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(colbase + c0);
+        const unsigned lane_base = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)c0;
         int done = 0, b = 0, since = 0;
         unsigned bph = 0;
         for (int i = 0; i < nst; ++i) {
             if (!mbar_wait(&acc_full[b], bph, p.err)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned ta = lane_base + (unsigned)(2 * b * p.N);
+            const unsigned ta = lane_base + (unsigned)(2 * b * p.TR0);
             // 16 columns of both slots per tcgen05.ld round (registers: the 64-column form has 32 per thread)
 #pragma unroll
             for (int g0 = 0; g0 < HALF; g0 += 16) {
@@ -303,7 +288,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
                 for (int g = 0; g < 16; g += 8)
                     if (g0 + g < ncols) {
                         ld8(r + g, ta + g0 + g);
-                        ld8(rx + g, ta + p.N + g0 + g);
+                        ld8(rx + g, ta + p.TR0 + g0 + g);
                     }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -325,7 +310,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
         for (int j = 0; j < HALF; ++j) acc[j] += (double)fs[j];
         (void)done;
         if (orow >= 0) {
-            double* out = partials + ((size_t)blockIdx.x * p.P + slab) * (p.m + p.mt) * p.m + (size_t)orow * p.m;
+            double* out = partials + (size_t)blockIdx.x * (p.m + p.mt) * p.m + (size_t)orow * p.m;
 #pragma unroll
             for (int j = 0; j < HALF; ++j)
                 if (c0 + j < p.m) out[c0 + j] = acc[j];
@@ -362,15 +347,14 @@ void make_rows_map(CUtensorMap* map, const float* base, long long F, int rows) {
 
 }  // namespace
 
-// Two 32-point slabs per stage when S and T fit 32-row blocks (m, mt <= 32): the 128-row A tile holds
-// S(slab 0), S(slab 1), T(slab 0), T(slab 1) at rows 0, 32, 64, 96, and B is its first 64 rows, so one
-// MMA serves both slabs (the cross-slab blocks of D are never read) and each slab writes its own
-// partials. Otherwise one slab per stage: S at row 0, T at row round8(m).
-static int slabs_for(int m, int mt) { return (((m + 7) & ~7) <= 32 && ((mt + 7) & ~7) <= 32) ? 2 : 1; }
+int gram_tc_blocks() { return sm_count(); }
 
-int gram_tc_blocks(int m, int mt) { return sm_count() * slabs_for(m, mt); }
+// Where the mixed form takes this kernel: blocks beyond one CUDA-core piece, which it then beats (m = mt = 60 on 128^3: 356 us
+// against 540 in pieces, in a solve). Within one piece the CUDA cores read every field once too, are limited by it and round
+// to nearest (m = mt = 24 on 95^3: 49.5 us against 74 here, with errors of 1e-8 against 2e-7).
+bool gram_tc_wins(int m, int mt) { return m > 32 || mt > 32; }
 
-// partials: [gram_tc_blocks(m, mt)][(m + mt) x m] of D = [S | T]^T S
+// partials: [gram_tc_blocks()][(m + mt) x m] of D = [S | T]^T S
 void launch_gram_tc(long long F, int m, const float* S, int mt, const float* T, double* partials, cudaStream_t s) {
     if (m < 1 || mt < 1 || ((m + 7) & ~7) + mt > ROWS || m > 64) throw std::invalid_argument("gram_tc: need m <= 64 and round8(m) + mt <= 128");
     if (F % 4 != 0) throw std::invalid_argument("gram_tc: F must be a multiple of 4");
@@ -381,17 +365,11 @@ void launch_gram_tc(long long F, int m, const float* S, int mt, const float* T, 
     p.F = F;
     p.m = m;
     p.mt = mt;
-    p.P = slabs_for(m, mt);
     const int m8 = (m + 7) & ~7, mt8 = (mt + 7) & ~7;
-    if (p.P == 2) {
-        p.SB = 32; p.TR0 = 64; p.TB = 32; p.N = 64; p.rows = 96 + mt8;
-        p.tbytes = TILE_BYTES;
-    } else {
-        p.SB = 0; p.TR0 = m8; p.TB = 0; p.N = m8; p.rows = m8 + mt8;
-        p.tbytes = p.rows * KT * 4;
-    }
-    const long long slab_pts = (long long)KT * p.P;
-    p.stages_total = (int)((F + slab_pts - 1) / slab_pts);
+    p.TR0 = m8;
+    p.rows = m8 + mt8;
+    p.tbytes = p.rows * KT * 4;
+    p.stages_total = (int)((F + KT - 1) / KT);
     // dynamic shared memory: two rings, the zero tail, 1 KB of alignment slack; the static barriers
     // take the last KB of the 227 KB a CTA may use
     constexpr int SMEM_BUDGET = 227 * 1024 - 1024;

@@ -113,8 +113,8 @@ int stencil_ctas(const Layout& L, int count);
 void launch_finish(const double* partials, int blocks, int nvals, double scale, double* out, cudaStream_t s);
 // the same for a rows x cols matrix of values, written transposed (out[c*rows + r])
 void launch_finish_transposed(const double* partials, int blocks, int rows, int cols, double scale, double* out, cudaStream_t s);
-// Two finishes in one launch, each value summed exactly as launch_finish / launch_finish_transposed would (bitwise):
-// trows > 0 writes value r*tcols + c to out[c*trows + r].
+// Two finishes in one launch (b may be empty), each value's partials summed in one fixed order: trows > 0 writes value
+// r*tcols + c to out[c*trows + r].
 struct FinishDesc {
     const double* partials = nullptr;
     int blocks = 0, nvals = 0;
@@ -123,9 +123,10 @@ struct FinishDesc {
     int trows = 0, tcols = 0;
 };
 void launch_finish_pair(const FinishDesc& a, const FinishDesc& b, cudaStream_t s);
-// G = S^T [S | T] on the tensor cores (k_gram_tc.cu): partials [gram_tc_blocks(m, mt)][(m + mt) x m] of the
+// G = S^T [S | T] on the tensor cores (k_gram_tc.cu): partials [gram_tc_blocks()][(m + mt) x m] of the
 // transpose D = [S | T]^T S; m <= 64, round8(m) + mt <= 128.
-int gram_tc_blocks(int m, int mt);
+int gram_tc_blocks();
+bool gram_tc_wins(int m, int mt);  // where the mixed form uses it: blocks beyond one CUDA-core piece
 void launch_gram_tc(long long F, int m, const float* S, int mt, const float* T, double* partials, cudaStream_t s);
 int reduce_blocks(long long F);
 // out-of-place dot products: partials [blocks][npairs] of sum a_p*b_p over F floats.
@@ -136,10 +137,11 @@ struct Pairs {
     const float* b[MAX];
 };
 void launch_dots(long long F, const Pairs& p, double* partials, int blocks, cudaStream_t s);
-// G = S^T [S | T] on CUDA cores: S m fields, T mt fields (both blocks stride F); partials [gram_blocks(m, mt)][m*(m+mt)]
-// row-major (row i = S_i, column j < m = S_j, j >= m = T_{j-m}). Returns the number of partial blocks written.
-int gram_blocks(int m, int mt);
-int launch_gram(long long F, int m, const float* S, int mt, const float* T, double* partials, cudaStream_t s);
+// G = S^T [S | T] on CUDA cores: S m fields, T mt fields (both blocks stride F); partials [gram_blocks(F)][m*(m+mt)]
+// row-major (row i = S_i, column j < m = S_j, j >= m = T_{j-m}). Returns the number of partial blocks written. lower (m ==
+// mt, else ignored): entries of S^T T above the diagonal may be left undefined.
+int gram_blocks(long long F);
+int launch_gram(long long F, int m, const float* S, int mt, const float* T, double* partials, cudaStream_t s, bool lower = false);
 // multipole moments Q_lm = sum rho R_lm(r) (l <= 6, Racah real solid harmonics, crates/qm/src/poisson.rs:89-120)
 void launch_moments(const Layout& L, const float* rho, double* partials, int blocks, cudaStream_t s);
 // max |f| over the six outer planes of the box -> partials [blocks] (max, finished by launch_finish_max)

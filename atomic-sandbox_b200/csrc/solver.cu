@@ -424,11 +424,11 @@ void Reducer::dots(const std::vector<std::pair<const float*, const float*>>& pai
     }
 }
 
-void Reducer::gram(int m, const float* S, int mt, const float* T, int off, double scale, const FinishDesc* extra) {
-    if (gram_mode == 1) {
+void Reducer::gram(int m, const float* S, int mt, const float* T, int off, double scale, const FinishDesc* extra, bool lower) {
+    if (gram_mode == 1 && gram_tc_wins(m, mt)) {
         // tensor cores: partials of D = [S | T]^T S, finished transposed into G = S^T [S | T]
         if (m > 64 || ((m + 7) & ~7) + mt > 128) throw std::invalid_argument("tensor-core Gram: block too large (m <= 64, round8(m) + mt <= 128)");
-        const int blocks = gram_tc_blocks(m, mt);
+        const int blocks = gram_tc_blocks();
         const size_t need = (size_t)blocks * m * (m + mt);
         if (need * sizeof(double) > partials_.bytes) partials_.alloc(need * sizeof(double));
         auto run = [&] { launch_gram_tc(L_.F, m, S, mt, T, partials_.d(), s_); };
@@ -449,10 +449,10 @@ void Reducer::gram(int m, const float* S, int mt, const float* T, int off, doubl
         }
         return;
     }
-    const int gblocks = gram_blocks(m, mt);
+    const int gblocks = gram_blocks(L_.F);
     const size_t need = (size_t)gblocks * m * (m + mt);
     if (need * sizeof(double) > partials_.bytes) partials_.alloc(need * sizeof(double));
-    auto run = [&] { launch_gram(L_.F, m, S, mt, T, partials_.d(), s_); };
+    auto run = [&] { launch_gram(L_.F, m, S, mt, T, partials_.d(), s_, lower); };
     if (timer) timer->time(KS_K_GRAM, m, mt, 4.0 * (m + mt) * L_.interior(), s_, run);
     else run();
     if (extra) {
@@ -911,7 +911,7 @@ void Solver::ensure_channel(int spin, int k) {
 void Solver::gram_checked(Reducer& red, int m, const float* S, int mt, const float* T, const FinishDesc* extra) {
     red.gram_mode = opt_.gram_mode;
     red.timer = &timer_;
-    red.gram(m, S, mt, T, 0, L_.h * L_.h * L_.h, extra);  // the L2 product <a, b> = h^3 sum a b
+    red.gram(m, S, mt, T, 0, L_.h * L_.h * L_.h, extra, true);  // the L2 product <a, b> = h^3 sum a b
 }
 
 EigenStats Solver::lobpcg(Channel& ch, Lane& lane, const float* V, double tol, double guess_tol, int max_iter, int head,

@@ -91,7 +91,8 @@ public:
     // sum_p a_p b_p * scale for every pair, written to res()[off + i]
     void dots(const std::vector<std::pair<const float*, const float*>>& pairs, int off, double scale);
     // G = scale * S^T [S | T], written to res()[off...] row-major m x (m + mt)
-    void gram(int m, const float* S, int mt, const float* T, int off, double scale = 1.0, const FinishDesc* extra = nullptr);
+    // (lower: only what a Rayleigh-Ritz step reads, S^T S and the lower triangle of S^T T)
+    void gram(int m, const float* S, int mt, const float* T, int off, double scale = 1.0, const FinishDesc* extra = nullptr, bool lower = false);
     double* res() const { return res_.d(); }
     double* partials() const { return partials_.d(); }
     int blocks() const { return blocks_; }
@@ -105,7 +106,7 @@ public:
     Faults* faults = nullptr;
     int readbacks = 0;
     double wait_s = 0;  // host time blocked in read()
-    int gram_mode = 0;  // 0: CUDA-core f32 Gram, 1: tensor-core 3xTF32 Gram
+    int gram_mode = 0;  // 0: CUDA-core f32 Gram, 1: tensor-core 3xTF32 Gram for the blocks where it is the faster one
     KernelTimer* timer = nullptr;  // times the Gram launch when set
     double* host() const { return host_; }
     static constexpr int RES_CAP = 1 << 16;

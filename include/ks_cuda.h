@@ -54,7 +54,8 @@ typedef struct {
 
 /* Solver construction options (no reference counterpart: B200 choices). */
 typedef struct {
-    int gram_mode;     /* LOBPCG Gram: 0 = FP32 CUDA cores ("plain FP32"), 1 = tensor cores (3xTF32, "mixed") */
+    int gram_mode;     /* LOBPCG Gram: 0 = FP32 CUDA cores ("plain FP32"), 1 = tensor cores (3xTF32, "mixed") for blocks of more
+                          than 32 columns, where they are the faster ones; smaller blocks take the CUDA cores */
     int n_extra;       /* extra LOBPCG bands per occupied spin channel (buffer columns, not occupied) */
     int init_mode;     /* cold orbitals: 0 = the reference's initial_orbitals (crates/qm/src/scf.rs:636-644), 1 = uniform(-1,1) */
     int reserved;

@@ -34,3 +34,24 @@ def test_block_update_over_solves(ks, oracle, n, k):
     for i in range(k):
         r = oracle.hamiltonian(n, h, xs[i], v) - ev[i] * xs[i]
         assert np.sqrt((r * r).sum() / (xs[i] * xs[i]).sum()) < tol * max(1.0, abs(ev[i])) + 63 * U * hnorm, (i, it)
+
+
+@pytest.mark.parametrize("n,m,mt", [(5, 1, 1), (9, 8, 8), (17, 9, 7), (29, 24, 24), (25, 17, 32), (33, 32, 32), (13, 33, 1), (13, 8, 33), (29, 8, 120),
+                                    (25, 12, 40), (25, 20, 60), (17, 40, 8), (21, 60, 60), (33, 33, 33)])
+@pytest.mark.parametrize("gram_mode", [0, 1])
+def test_gram_pieces_match_f64(ks, n, m, mt, gram_mode):
+    """S^T [S | T] with one piece and with several (more than 32 rows or columns), every count of row and column groups of
+    8, in both forms. Products of one warp's points are summed in f32, two chains of 16 and then one over its slabs (3 at
+    most here), the rest in f64: |error| <= (16 + 1 + 3) U |s| |t| by Cauchy-Schwarz; the tensor cores' 3xTF32 form
+    (blocks beyond one piece) keeps 2e-6."""
+    if gram_mode == 1 and ((m + 7) // 8 * 8 + mt > 128 or m > 64):
+        pytest.skip("beyond the tensor-core form's block")
+    rng = np.random.default_rng(m + mt)
+    s, t = f32(rng.standard_normal((m, n ** 3))), f32(rng.standard_normal((mt, n ** 3)))
+    g = ks.gram(n, s, t, gram_mode=gram_mode)
+    st = np.concatenate([s, t])
+    scale = np.sqrt(np.outer((s * s).sum(1), (st * st).sum(1)))
+    err = (np.abs(g - s @ st.T) / scale).max()
+    assert err < (2e-6 if gram_mode == 1 and (m > 32 or mt > 32) else 20 * U), err
+    if gram_mode == 0:
+        assert np.array_equal(g[:, :m], g[:, :m].T)
