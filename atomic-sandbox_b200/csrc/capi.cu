@@ -510,7 +510,7 @@ ks_status ks_apply_hamiltonian(int n, double h, int count, const double* psi, co
         sc.upload_fields(v, 1, vv);
         StencilArgs a;
         a.mode = ST_HAMILTONIAN;
-        a.scale = (float)(-0.5 / (h * h));
+        a.scale = -0.5 / (h * h);
         a.V = vv.at(0);
         launch_stencil(sc.L, x.tmap, count, a, o.at(0), sc.s);
         sc.download_fields(o.at(0), count, out);
@@ -528,7 +528,7 @@ ks_status ks_apply_laplacian(int n, double h, const double* f, double* out) {
         sc.upload_fields(f, 1, x);
         StencilArgs a;
         a.mode = ST_LAPLACIAN;
-        a.scale = (float)(1.0 / (h * h));
+        a.scale = 1.0 / (h * h);
         launch_stencil(sc.L, x.tmap, 1, a, o.at(0), sc.s);
         sc.download_fields(o.at(0), 1, out);
         return KS_OK;
@@ -552,7 +552,7 @@ ks_status ks_apply_precond(int n, double h, const double* v, double lambda, cons
                                 hx.at(0), q.at(0), part.d(), reduce_blocks(sc.L.F), sc.s);
         StencilArgs jac;
         jac.mode = ST_JACOBI;
-        jac.scale = (float)(-0.5 / (h * h));
+        jac.scale = -0.5 / (h * h);
         jac.V = vv.at(0);
         jac.R = rr.at(0);
         jac.lambda = th.d() + 1;
@@ -739,7 +739,7 @@ ks_status ks_autotune_stencil(int n, const int* counts, int ncount, int* chunks_
             for (int mi = 0; mi < 2; ++mi) {
                 StencilArgs a;
                 a.mode = mi == 0 ? ST_HAMILTONIAN : ST_JACOBI;
-                a.scale = (float)(-0.5 / (h * h));
+                a.scale = -0.5 / (h * h);
                 a.V = v.at(0);
                 if (a.mode == ST_JACOBI) {
                     a.R = r.at(0);
@@ -981,7 +981,7 @@ ks_status ks_hpsi_device(void* stream, int n, double h, int count, const float* 
         }
         StencilArgs a;
         a.mode = ST_HAMILTONIAN;
-        a.scale = (float)(-0.5 / (h * h));
+        a.scale = -0.5 / (h * h);
         a.V = v;
         launch_stencil(L, map, count, a, out, static_cast<cudaStream_t>(stream));
         return KS_OK;

@@ -3,24 +3,23 @@
 //
 // Reference operators: crates/qm/src/stencil.rs:21-51 (coefficients c = [-205/72, 8/5, -1/5,
 // 8/315, -1/560], Dirichlet zero outside the box), crates/qm-gpu/src/shaders/stencil.wgsl:58-106
-// (hamiltonian, jacobi_step). The centre is folded into second differences,
-//     lap f = s sum_{m=1..4} c_m sum_axes [(f_{+m} - f_0) + (f_{-m} - f_0)],
-// exact in real arithmetic because c_0 = -2 sum c_m, and exact per difference in f32 for smooth f (the
-// differences carry no rounding, which keeps the f32 residual floor of the reference's stop rules). s is the
-// operator's scale (1/h^2, or -1/(2 h^2) for H); smallest coefficients first.
+// (hamiltonian, jacobi_step). The centre is folded into differences of neighbours (below), exact in real arithmetic
+// because c_0 = -2 sum c_m, and exact per difference in f32 for smooth f, which keeps the f32 residual floor of the
+// reference's stop rules. The operator's scale (1/h^2, or -1/(2 h^2) for H) multiplies the sum.
 //
-// B200 design ("2.5-D" tiling): a CTA owns a 32 x 16 (x, y) tile of one field and marches a z-chunk. Each z-plane
-// of the tile plus its 4-point xy halo (40 x 24 floats) is staged in shared memory by one TMA load
-// (cp.async.bulk.tensor.4d); the tensor map's extent is n on every axis, so the halo beyond the box arrives as the
-// hardware's zero fill -- the Dirichlet boundary costs no branches and no ghost storage. An 8-deep ring of planes
-// keeps four planes of prefetch in flight. Each of the 128 threads owns four consecutive x-outputs of one row: it
-// reads its centre, x- and y-neighbours as 16-byte quads (11 shared loads per 4 outputs), keeps the nine z-values of
-// its quad in a register queue that moves up one plane per step, and computes the two packed pairs of the quad with
-// Blackwell's f32x2 arithmetic. A neighbour pair that straddles two quads (odd x offsets) is differenced with two
-// scalar subtractions instead of being repacked. The V / R reads (cp.async copies one plane ahead into a small shared
-// ring) and the stores are coalesced 16-byte accesses;
-// the quad's pad columns are stored as 0. Measured against the 2 x 2-outputs-per-thread form it replaces: the same
-// outputs bit for bit at h = 0.25, and H psi on 95^3 at 8 / 16 / 64 vectors 13 / 13 / 21 % faster.
+// B200 design ("2.5-D" tiling): a CTA owns a BX x 16 (x, y) tile of one field and marches a z-chunk. Each z-plane
+// of the tile plus its 4-point xy halo is staged in shared memory by one TMA load (cp.async.bulk.tensor.4d); the tensor
+// map's extent is n on every axis, so the halo beyond the box arrives as the hardware's zero fill -- the Dirichlet
+// boundary costs no branches and no ghost storage. A ring of 8 planes keeps up to four planes of prefetch in flight.
+// Each thread owns four consecutive x-outputs of two adjacent rows: it reads its centre, x- and y-neighbours as 16-byte
+// quads (13 shared loads per 8 outputs, the ten y-rows serving both output rows) and works on packed pairs with
+// Blackwell's f32x2 arithmetic. The z-direction holds no queue of planes: a new plane's second difference is added to the
+// seven outputs it belongs to (ZRow), so nothing moves between registers. The V / R reads (cp.async copies one plane ahead
+// into a small shared ring) and the stores are coalesced 16-byte accesses; the quad's pad columns are stored as 0.
+//
+// What bounds it: instruction issue. With one row per thread, a nine-deep register queue in z and symmetric differences
+// (the form this replaces) 128 outputs took 230 warp instructions, 32 of them register moves. Measured per launch, before and after: H psi on 95^3 x 16 vectors 43.0 -> 34.9 us,
+// on 128^3 x 40 216 -> 170 us, on 48^3 x 8 8.3 -> 7.2 us, a sweep on 128^3 x 20 in a solve 160 -> 125 us.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -35,31 +34,36 @@ namespace {
 
 typedef unsigned long long u64;
 
-constexpr int BX = 32, BY = 16;
-constexpr int HXW = BX + 8, HYW = BY + 8;          // staged plane with halo: 40 x 24
-constexpr int NS = 8;                               // ring depth (planes)
-constexpr int PLANE_FLOATS = HXW * HYW;             // 960
-constexpr unsigned PLANE_BYTES = PLANE_FLOATS * 4;  // 3840 = 30 * 128
-constexpr int THREADS = 128;                        // 8 x-quads * 16 rows
-// The TMA rules the plane loads rely on, checked here because a violation faults the GPU instead of returning an
-// error: the box's inner extent is a multiple of 16 bytes; a load's x coordinate, x0 - 4 with x0 a multiple of BX,
-// times 4 bytes is a multiple of 16 (negative x is allowed for loads and reads the zero fill); each ring plane starts
-// on a 128-byte boundary. The quads the threads read start on 16-byte boundaries: rows of HXW floats, quads at
-// 4 * tx + 4 (and +-4 for the x-neighbours). The z-queue issues plane s + 12 into the buffer plane s + 4 left, which
-// needs NS = 8.
-static_assert((HXW * 4) % 16 == 0, "TMA box inner extent must be a multiple of 16 bytes");
-static_assert((BX * 4) % 16 == 0 && (4 * 4) % 16 == 0, "TMA x coordinate x0 - 4 must be a multiple of 16 bytes");
-static_assert(PLANE_BYTES % 128 == 0, "ring planes must start on 128-byte boundaries");
-static_assert(NS == 8, "plane s + 12 reuses the buffer of plane s + 4 only with an 8-deep ring");
-static_assert(THREADS == (BX / 4) * BY, "one thread per x-quad of a row");
-// resident CTAs per SM: registers capped at 96 per thread (no spills) for 20 warps per SM; 4 and 6 CTAs per SM
-// measured slower (H psi on 95^3: 4 CTAs 182 us at 64 vectors, 6 CTAs 144 us, against 137 us at 5)
-constexpr int CTAS_PER_SM = 5;
+constexpr int BY = 16;                              // tile rows
+constexpr int HYW = BY + 8;
+constexpr int ROWS = 2;                             // adjacent rows per thread
+// A tile of BX columns: the staged plane with its halo, and one thread per x-quad and row pair. 12 warps per SM in every
+// width (registers capped at 168 per thread): 6 CTAs of 64 threads, 4 of 96 or 3 of 128.
+template <int BX>
+struct Tile {
+    static constexpr int HXW = BX + 8;
+    static constexpr int QX = BX / 4;
+    static constexpr int THREADS = QX * (BY / ROWS);
+    static constexpr int PLANE_FLOATS = HXW * HYW;
+    static constexpr unsigned PLANE_BYTES = PLANE_FLOATS * 4;
+    static constexpr int CTAS_PER_SM = 12 * 32 / THREADS;
+    // The TMA rules the plane loads rely on, checked here because a violation faults the GPU instead of returning an
+    // error: the box's inner extent is a multiple of 16 bytes; a load's x coordinate, x0 - 4 with x0 a multiple of BX,
+    // times 4 bytes is a multiple of 16 (negative x is allowed for loads and reads the zero fill); each ring plane starts
+    // on a 128-byte boundary. The quads the threads read start on 16-byte boundaries: rows of HXW floats, quads at
+    // 4 * tx + 4 (and +-4 for the x-neighbours).
+    static_assert((HXW * 4) % 16 == 0, "TMA box inner extent must be a multiple of 16 bytes");
+    static_assert((BX * 4) % 16 == 0 && (4 * 4) % 16 == 0, "TMA x coordinate x0 - 4 must be a multiple of 16 bytes");
+    static_assert(PLANE_BYTES % 128 == 0, "ring planes must start on 128-byte boundaries");
+    static_assert(THREADS % 32 == 0, "whole warps");
+};
+// ring depth in planes: a step reads planes s + 4 (the centre) and s + 8 (the newest), so five planes are live and the
+// others in flight. The Jacobi mode's larger side ring leaves room for 7.
+template <int MODE>
+constexpr int ring_depth() { return MODE == ST_JACOBI ? 7 : 8; }
 // The per-plane global reads of a step (V; r and the stored factor in the Jacobi mode) are staged one plane ahead by
 // per-thread cp.async copies into a 2-deep shared "side" ring (12 KB per CTA in the Jacobi mode, 4 KB for H and the
-// residual form), so their latency runs behind the previous plane's arithmetic without holding registers. Against
-// register loads at the step that uses them: the H2O 95^3 solve 176.5 -> 172.3 ms, Jacobi sweep 34.0 -> 33.0 us,
-// bitwise-identical results. Three planes ahead, or V left to the L2 in the Jacobi mode, measured slower.
+// residual form), so their latency runs behind the previous plane's arithmetic without holding registers.
 constexpr int SD = 2;
 template <int MODE>
 constexpr int n_side() { return MODE == ST_JACOBI ? 3 : (MODE == ST_LAPLACIAN ? 0 : 1); }
@@ -72,17 +76,28 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 constexpr long long WAIT_LIMIT = 1LL << 22;         // bounded mbarrier waits (~seconds)
 constexpr long long DRAIN_LIMIT = 1LL << 16;        // waits for copies in flight after a wait gave up
 
-constexpr float C1 = 1.6f, C2 = -0.2f, C3 = 0.025396825396825397f, C4 = -0.0017857142857142857f;
-#ifndef KS_FOLD_SCALE
-#define KS_FOLD_SCALE 0
-#endif
-constexpr bool FOLD_SCALE = KS_FOLD_SCALE != 0;
+// The 8th-order second difference sum_m c_m (f_m - 2 f_0 + f_-m) on the first differences e_j = f_j+1 - f_j
+//     sum_{j=0..3} b_j (e_j - e_-1-j),  b_j = sum_{m > j} c_m   (x and y)
+// and on the second differences s_i = e_i - e_i-1
+//     sum_{|i| <= 3} g_|i| s_i,         g_i = sum_{j >= i} b_j  (z).
+// kappa is free in exact arithmetic: the coefficients are divided by it and the operator's scale multiplied. It is the
+// f32 value in [1, 2) for which the rounded coefficients come closest to the exact ones in the operator's second moment
+// (what a smooth field sees: sum_j (2j + 1) b_j and g_0 + 2 (g_1 + g_2 + g_3) are off by 4e-11) and in b_0, b_1, g_0, g_1; the
+// plain c_m rounded to f32 are off by up to 8e-8. The scale is applied as an f32 pair hi + lo, so 1/h^2 is not rounded
+// to f32 either. Against 64 bits the operator's error is 0.82 .. 1.06 of the direct difference form's
+// sum_m c_m [(f_m - f_0) + (f_-m - f_0)] over h = 0.18 .. 0.30, smooth and rough fields (0.93 in the mean).
+constexpr double KAPPA = 1.6073455810546875;
+constexpr double C1 = 8.0 / 5.0, C2 = -1.0 / 5.0, C3 = 8.0 / 315.0, C4 = -1.0 / 560.0;
+constexpr double B3D = C4, B2D = C3 + B3D, B1D = C2 + B2D, B0D = C1 + B1D;
+constexpr double G2D = B2D + B3D, G1D = B1D + G2D, G0D = B0D + G1D;
+constexpr float CB0 = (float)(B0D / KAPPA), CB1 = (float)(B1D / KAPPA), CB2 = (float)(B2D / KAPPA), CB3 = (float)(B3D / KAPPA);
+constexpr float CG0 = (float)(G0D / KAPPA), CG1 = (float)(G1D / KAPPA), CG2 = (float)(G2D / KAPPA);
 
 struct Params {
     int n, P;
     long long F;
     int tiles_x, tiles_y, zc;
-    float scale, omega, diag_t;
+    float scale_hi, scale_lo, omega, diag_t;
     const float* V;
     const float* R;
     const double* lambda;
@@ -132,6 +147,12 @@ __device__ __forceinline__ void tma_load_plane(float* dst, const CUtensorMap* ma
         : "memory");
 }
 
+// Before a TMA load refills a ring slot: the barrier orders the CTA's reads of the slot before this thread, the fence
+// orders them before the load's writes, which are the async proxy's. Without it reads that were still in flight when
+// the barrier released thread 0 could see the new plane: with kernels of three streams on the chip, solves stopped
+// being bit for bit reproducible.
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 // ---- packed f32x2 arithmetic (sm_100): one instruction for two x-neighbours
 __device__ __forceinline__ u64 add2(u64 a, u64 b) { u64 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ u64 sub2(u64 a, u64 b) { u64 d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
@@ -148,64 +169,86 @@ __device__ __forceinline__ u64 pk(float lo, float hi) {
 }
 __device__ __forceinline__ float lo_of(u64 v) { return __uint_as_float((unsigned)v); }
 __device__ __forceinline__ float hi_of(u64 v) { return __uint_as_float((unsigned)(v >> 32)); }
-__device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-// (a0 - f0.lo, a1 - f0.hi)
-__device__ __forceinline__ u64 dif(float a0, float a1, u64 f0) { return sub2(pk(a0, a1), f0); }
+// four x-consecutive values as two packed pairs
+struct Quad { u64 a, b; };
+__device__ __forceinline__ Quad ldq(const float* p) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return {v.x, v.y};
+}
+__device__ __forceinline__ Quad ldq(const float4* p) { return ldq(reinterpret_cast<const float*>(p)); }
+__device__ __forceinline__ Quad operator-(const Quad& x, const Quad& y) { return {sub2(x.a, y.a), sub2(x.b, y.b)}; }
+__device__ __forceinline__ Quad operator+(const Quad& x, const Quad& y) { return {add2(x.a, y.a), add2(x.b, y.b)}; }
+__device__ __forceinline__ Quad fmaq(u64 k, const Quad& x, const Quad& y) { return {fma2(k, x.a, y.a), fma2(k, x.b, y.b)}; }
+__device__ __forceinline__ Quad mulq(u64 k, const Quad& x) { return {mul2(k, x.a), mul2(k, x.b)}; }
+__device__ __forceinline__ Quad fmaq(const Quad& x, const Quad& y, const Quad& z) { return {fma2(x.a, y.a, z.a), fma2(x.b, y.b, z.b)}; }
+__device__ __forceinline__ u64 rep(float v) { return pk(v, v); }
+// (v, v) kept in a register pair: the compiler would rather rebuild a constant pair at every use
+__device__ __forceinline__ u64 rep_kept(float v) {
+    u64 d;
+    asm volatile("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
+    return d;
+}
+struct Pairs { u64 b0, b1, b2, b3, g0, g1, g2, hi, lo; };  // the coefficients (g_3 = b_3) and the scale, as (k, k)
 
-// sum_m (c_m s) d_m of the thread's quad, as two packed pairs (x0, x0+1) and (x0+2, x0+3). cpl: the quad's address
-// in the centre plane (x-neighbour quads at -4 / +4, y-neighbours at +-m*HXW); q: the z-queue, q[4] the centre.
-// The y-neighbour quads are loaded inside the m loop, largest m first, so that only two are live at a time.
-__device__ __forceinline__ void lap_quad(const float* cpl, const float4 (&q)[9], const u64 (&k)[5], u64& o0, u64& o1) {
-    const float4 c = q[4];
-    const float4 l = lds4(cpl - 4), r = lds4(cpl + 4);
-    const float xs[12] = {l.x, l.y, l.z, l.w, c.x, c.y, c.z, c.w, r.x, r.y, r.z, r.w};
-    const u64 f0[2] = {pk(c.x, c.y), pk(c.z, c.w)};
-    u64 acc[2];
-#pragma unroll
-    for (int m = 4; m >= 1; --m) {
-        const float4 yu = lds4(cpl + m * HXW), yd = lds4(cpl - m * HXW);
-        const float4& zu = q[4 + m];
-        const float4& zd = q[4 - m];
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const int b = 4 + 2 * p;  // the pair's first element in xs
-            u64 dx;
-            if (m & 1) {
-                // odd offsets straddle two quads: two scalar differences instead of a repacked pair
-                const float a0 = xs[b + m] - lo_of(f0[p]), a1 = xs[b + 1 + m] - hi_of(f0[p]);
-                const float b0 = xs[b - m] - lo_of(f0[p]), b1 = xs[b + 1 - m] - hi_of(f0[p]);
-                dx = add2(pk(a0, a1), pk(b0, b1));
-            } else {
-                dx = add2(dif(xs[b + m], xs[b + 1 + m], f0[p]), dif(xs[b - m], xs[b + 1 - m], f0[p]));
-            }
-            u64 dy, dz;
-            if (p == 0) {
-                dy = add2(dif(yu.x, yu.y, f0[0]), dif(yd.x, yd.y, f0[0]));
-                dz = add2(dif(zu.x, zu.y, f0[0]), dif(zd.x, zd.y, f0[0]));
-            } else {
-                dy = add2(dif(yu.z, yu.w, f0[1]), dif(yd.z, yd.w, f0[1]));
-                dz = add2(dif(zu.z, zu.w, f0[1]), dif(zd.z, zd.w, f0[1]));
-            }
-            const u64 d = add2(add2(dx, dy), dz);
-            acc[p] = (m == 4) ? mul2(k[4], d) : fma2(k[m], d, acc[p]);
-        }
+// One row's z direction: the sums of the six output planes still open, the last value and the last first difference.
+// A plane's second difference is added to the seven outputs it belongs to as it becomes known, each sum moving to its
+// neighbour's register in the same FMA, so the march needs no queue of values and no register moves.
+struct ZRow {
+    Quad p0, p1, p2, p3, p4, p5, f, e;
+    __device__ __forceinline__ void start(const Quad& f0, const Quad& f1) {
+        const Quad z = {0, 0};
+        p0 = p1 = p2 = p3 = p4 = p5 = z;
+        e = f1 - f0;
+        f = f1;
     }
-    o0 = acc[0];
-    o1 = acc[1];
+    // the next plane's values in, the finished sum of the plane four below out
+    __device__ __forceinline__ Quad push(const Quad& fn, const Pairs& k) {
+        const Quad en = fn - f, s = en - e;
+        f = fn;
+        e = en;
+        const Quad done = fmaq(k.b3, s, p0);
+        p0 = fmaq(k.g2, s, p1);
+        p1 = fmaq(k.g1, s, p2);
+        p2 = fmaq(k.g0, s, p3);
+        p3 = fmaq(k.g1, s, p4);
+        p4 = fmaq(k.g2, s, p5);
+        p5 = mulq(k.b3, s);
+        return done;
+    }
+};
+
+// the x direction's e_j - e_-1-j, j = 0..3, of the quad c between its neighbour quads l and r. The pairs of odd offsets
+// straddle two registers, so these are scalar subtractions, each difference shared by the outputs it belongs to.
+__device__ __forceinline__ void x_terms(const Quad& l, const Quad& c, const Quad& r, Quad (&d)[4]) {
+    const float xs[12] = {lo_of(l.a), hi_of(l.a), lo_of(l.b), hi_of(l.b), lo_of(c.a), hi_of(c.a),
+                          lo_of(c.b), hi_of(c.b), lo_of(r.a), hi_of(r.a), lo_of(r.b), hi_of(r.b)};
+    float e[11];
+#pragma unroll
+    for (int i = 0; i < 11; ++i) e[i] = xs[i + 1] - xs[i];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        d[j].a = pk(e[4 + j] - e[3 - j], e[5 + j] - e[4 - j]);
+        d[j].b = pk(e[6 + j] - e[5 - j], e[7 + j] - e[6 - j]);
+    }
 }
 
 // f64 sum of f0 * o over the valid elements of a quad (the Poisson p.Ap and the kinetic <psi, lap psi>)
-__device__ __forceinline__ double quad_dot(const float4& f, u64 o0, u64 o1, bool e1, bool e2, bool e3) {
-    double d = (double)f.x * (double)lo_of(o0);
-    if (e1) d += (double)f.y * (double)hi_of(o0);
-    if (e2) d += (double)f.z * (double)lo_of(o1);
-    if (e3) d += (double)f.w * (double)hi_of(o1);
+__device__ __forceinline__ double quad_dot(const Quad& f, const Quad& o, bool e1, bool e2, bool e3) {
+    double d = (double)lo_of(f.a) * (double)lo_of(o.a);
+    if (e1) d += (double)hi_of(f.a) * (double)hi_of(o.a);
+    if (e2) d += (double)lo_of(f.b) * (double)lo_of(o.b);
+    if (e3) d += (double)hi_of(f.b) * (double)hi_of(o.b);
     return d;
 }
+__device__ __forceinline__ void store_quad(float* dst, const Quad& o, bool e1, bool e2, bool e3) {
+    *reinterpret_cast<float4*>(dst) = make_float4(lo_of(o.a), e1 ? hi_of(o.a) : 0.f, e2 ? lo_of(o.b) : 0.f, e3 ? hi_of(o.b) : 0.f);
+}
 
-template <int MODE, bool DOT>
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) stencil_kernel(const __grid_constant__ CUtensorMap tmap, Params p, float* __restrict__ out) {
-    extern __shared__ __align__(1024) float ring[];  // NS planes of 40 x 24
+template <int MODE, bool DOT, int BX>
+__global__ void __launch_bounds__(Tile<BX>::THREADS, Tile<BX>::CTAS_PER_SM) stencil_kernel(const __grid_constant__ CUtensorMap tmap, Params p, float* __restrict__ out) {
+    constexpr int HXW = Tile<BX>::HXW, PLANE_FLOATS = Tile<BX>::PLANE_FLOATS, THREADS = Tile<BX>::THREADS, NS = ring_depth<MODE>();
+    constexpr unsigned PLANE_BYTES = Tile<BX>::PLANE_BYTES;
+    extern __shared__ __align__(1024) float ring[];  // NS planes of HXW x 24
     __shared__ __align__(8) uint64_t bar[NS];
 
     const int vec = blockIdx.y;
@@ -218,13 +261,13 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) stencil_kernel(const __g
     const int z0 = chunk * p.zc;
     const int nz = min(z0 + p.zc, p.n) - z0;
     const int nplanes = nz + 8;  // relative plane q <-> z = z0 - 4 + q
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
-    const int gx = x0 + 4 * tx, gy = y0 + ty;
+    const int tx = threadIdx.x % Tile<BX>::QX, ty = threadIdx.x / Tile<BX>::QX;
+    const int gx = x0 + 4 * tx, gy = y0 + ROWS * ty;
     // the quad's elements inside the box (gx is a multiple of 4 below n <= P, so the whole quad lies inside the
     // row's P floats; elements at or past n are pad columns and are stored as 0)
-    const bool ok = gx < p.n && gy < p.n;
+    const bool ok[ROWS] = {gx < p.n && gy < p.n, gx < p.n && gy + 1 < p.n};
     const bool e1 = gx + 1 < p.n, e2 = gx + 2 < p.n, e3 = gx + 3 < p.n;
-    const int ci = (ty + 4) * HXW + 4 * tx + 4;
+    const int ci = (ROWS * ty + 4) * HXW + 4 * tx + 4;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; ++i) mbar_init(&bar[i], 1);
@@ -243,153 +286,170 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) stencil_kernel(const __g
     if (threadIdx.x == 0)
         for (; issued < min(NS, nplanes); ++issued) issue(issued);
 
-    float4 q[9];
-    bool alive = true;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        alive = mbar_wait(&bar[i], 0, p.err, alive ? WAIT_LIMIT : 1) && alive;
-        q[i] = lds4(ring + i * PLANE_FLOATS + ci);
-    }
-    __syncthreads();  // planes 0..3 are consumed: their buffers take planes 8..11
-    if (alive && threadIdx.x == 0)
-        for (; issued < min(NS + 4, nplanes); ++issued) issue(issued);
-
-    // the coefficients; with FOLD_SCALE the operator's scale is folded into them, else it multiplies the sum (the
-    // same bits when the scale is a power of two)
-    u64 kc[5];
-    const float ks = FOLD_SCALE ? p.scale : 1.0f;
-    kc[0] = 0;
-    kc[1] = pk(C1 * ks, C1 * ks);
-    kc[2] = pk(C2 * ks, C2 * ks);
-    kc[3] = pk(C3 * ks, C3 * ks);
-    kc[4] = pk(C4 * ks, C4 * ks);
-    const u64 scale2 = pk(p.scale, p.scale);
-    const float lam = (MODE == ST_JACOBI || MODE == ST_HAM_RESIDUAL) ? (float)p.lambda[vec] : 0.0f;
-    // theta split into f32 hi + lo, as the residual kernel does: r = fma(-lo, x, fma(-hi, x, Hx))
-    const double th = (MODE == ST_HAM_RESIDUAL) ? p.theta[vec] : 0.0;
-    const float th_hi = (float)th, th_lo = (float)(th - (double)th_hi);
-    const long long plane = (long long)p.n * p.P;
-    const long long row0 = ((long long)z0 * p.n + gy) * p.P + gx;
+    // 32-bit offsets inside a field (F < 2^31) from per-vector bases: one address instruction per access
+    const int plane = p.n * p.P;
+    const int row0 = (z0 * p.n + gy) * p.P + gx;
     const long long vbase = (long long)vec * p.F;
-    const float* vrow = p.V ? p.V + row0 : nullptr;
-    const float* rrow = p.R ? p.R + vbase + row0 : nullptr;
-    float* orow = out + vbase + row0;
-    float* orow2 = (MODE == ST_HAM_RESIDUAL) ? p.out2 + vbase + row0 : nullptr;
-    float* drow = p.dinv ? p.dinv + vbase + row0 : nullptr;
-    // the side ring, [SD][NSIDE][THREADS] float4 after the plane ring: slot t % SD holds this thread's V (r, factor)
+    const float* rbase = p.R ? p.R + vbase : nullptr;
+    float* obase = out + vbase;
+    float* obase2 = (MODE == ST_HAM_RESIDUAL) ? p.out2 + vbase : nullptr;
+    float* dbase = p.dinv ? p.dinv + vbase : nullptr;
+    // the side ring, [SD][NSIDE][ROWS][THREADS] float4 after the plane ring: slot t % SD holds this thread's V (r, factor)
     // quads of output plane t. Each thread reads only its own copies, after its own wait_group, and refills a slot
     // only after the step that read it has consumed the values.
     constexpr int NSIDE = n_side<MODE>();
-    float4* side = reinterpret_cast<float4*>(ring + NS * PLANE_FLOATS);
-    auto side_issue = [&](int t) {
+    float4* side = reinterpret_cast<float4*>(ring + NS * PLANE_FLOATS) + threadIdx.x;
+    auto side_issue = [&](int t, int off) {
         if (NSIDE > 0) {
-            if (ok && t < nz) {
-                float4* dst = side + (t % SD) * NSIDE * THREADS + threadIdx.x;
-                cp_async16(dst, vrow + t * plane);
-                if (MODE == ST_JACOBI) {
-                    cp_async16(dst + THREADS, rrow + t * plane);
-                    if (drow) cp_async16(dst + 2 * THREADS, drow + t * plane);
-                }
+            if (t < nz) {
+                float4* dst = side + (t % SD) * NSIDE * ROWS * THREADS;
+#pragma unroll
+                for (int w = 0; w < ROWS; ++w)
+                    if (ok[w]) {
+                        cp_async16(dst + w * THREADS, p.V + (off + w * p.P));
+                        if (MODE == ST_JACOBI) {
+                            cp_async16(dst + (ROWS + w) * THREADS, rbase + (off + w * p.P));
+                            if (dbase) cp_async16(dst + (2 * ROWS + w) * THREADS, dbase + (off + w * p.P));
+                        }
+                    }
             }
             cp_async_commit();  // one group per plane, empty or not, so that wait_group counts planes
         }
     };
 #pragma unroll
-    for (int t = 0; t < SD - 1; ++t) side_issue(t);
+    for (int t = 0; t < SD - 1; ++t) side_issue(t, row0 + t * plane);
+
+    const Pairs k = {rep_kept(CB0), rep_kept(CB1), rep_kept(CB2), rep_kept(CB3), rep_kept(CG0), rep_kept(CG1), rep_kept(CG2),
+                     rep_kept(p.scale_hi), rep_kept(p.scale_lo)};
+    ZRow zr[ROWS];
+    bool alive = true;
+    auto plane_in = [&](int q) {  // planes 0..7 of the march's start
+        alive = mbar_wait(&bar[q % NS], (unsigned)((q / NS) & 1), p.err, alive ? WAIT_LIMIT : 1) && alive;
+        return ring + (q % NS) * PLANE_FLOATS + ci;
+    };
+    {
+        Quad f0[ROWS];
+        const float* at = plane_in(0);
+#pragma unroll
+        for (int w = 0; w < ROWS; ++w) f0[w] = ldq(at + w * HXW);
+        at = plane_in(1);
+#pragma unroll
+        for (int w = 0; w < ROWS; ++w) zr[w].start(f0[w], ldq(at + w * HXW));
+    }
+#pragma unroll
+    for (int i = 2; i < 8; ++i) {
+        if (i == 4) {
+            __syncthreads();  // planes 0..3 are consumed: their buffers take the next four
+            if (alive && threadIdx.x == 0) {
+                proxy_fence();
+                for (; issued < min(NS + 4, nplanes); ++issued) issue(issued);
+            }
+        }
+        const float* at = plane_in(i);
+#pragma unroll
+        for (int w = 0; w < ROWS; ++w) zr[w].push(ldq(at + w * HXW), k);
+    }
+
+    const float lam = (MODE == ST_JACOBI || MODE == ST_HAM_RESIDUAL) ? (float)p.lambda[vec] : 0.0f;
+    // theta split into f32 hi + lo, as the residual kernel does: r = fma(-lo, x, fma(-hi, x, Hx))
+    const double th = (MODE == ST_HAM_RESIDUAL) ? p.theta[vec] : 0.0;
+    const float th_hi = (float)th, th_lo = (float)(th - (double)th_hi);
     double dot = 0.0;
-    // the compact loop body (not unrolled): unrolled bodies measured slower (the instruction cache)
-#pragma unroll 1
-    for (int s = 0; s < nz; ++s) {
-        const int qn = s + 8;
-        alive = mbar_wait(&bar[qn % NS], (unsigned)((qn / NS) & 1), p.err, alive ? WAIT_LIMIT : 1) && alive;
-        q[8] = lds4(ring + (qn % NS) * PLANE_FLOATS + ci);
-        const float* cpl = ring + ((s + 4) % NS) * PLANE_FLOATS + ci;
+    // two steps per iteration where the side ring is read or two fields are stored (95^3 k = 8: the sweep 29.1 -> 28.3 us, the
+    // residual form 41.4 -> 39.8), one for H and the Laplacian, which gained nothing
+    constexpr int STEPS = MODE == ST_JACOBI || MODE == ST_HAM_RESIDUAL ? 2 : 1;
+    int sn = 8 % NS, sc = 4 % NS;  // ring slots of the newest and the centre plane
+    unsigned pn = (8 / NS) & 1;    // parity of the newest plane's round
+    int off = row0;
+#pragma unroll STEPS
+    for (int s = 0; s < nz; ++s, off += plane) {
+        alive = mbar_wait(&bar[sn], pn, p.err, alive ? WAIT_LIMIT : 1) && alive;
         // the next plane's side copies go out before this plane's are read
-        const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 v = zero4, r = zero4, dq = zero4;
-        if (NSIDE > 0) {
-            side_issue(s + SD - 1);
-            cp_async_wait<SD - 1>();
-            const float4* sl = side + (s % SD) * NSIDE * THREADS + threadIdx.x;
-            if (ok) v = sl[0];
-            if (MODE == ST_JACOBI && ok) r = sl[THREADS];
-            if (MODE == ST_JACOBI && ok && drow) dq = sl[2 * THREADS];
+        side_issue(s + SD - 1, off + (SD - 1) * plane);
+        const float* fresh = ring + sn * PLANE_FLOATS + ci;
+        const float* cpl = ring + sc * PLANE_FLOATS + ci;
+        Quad acc[ROWS], f[ROWS];
+#pragma unroll
+        for (int w = 0; w < ROWS; ++w) {
+            acc[w] = zr[w].push(ldq(fresh + w * HXW), k);
+            f[w] = ldq(cpl + w * HXW);
         }
-        u64 o0, o1;
-        lap_quad(cpl, q, kc, o0, o1);
-        if (!FOLD_SCALE) {
-            o0 = mul2(o0, scale2);
-            o1 = mul2(o1, scale2);
+        Quad dx[ROWS][4];
+#pragma unroll
+        for (int w = 0; w < ROWS; ++w) x_terms(ldq(cpl + w * HXW - 4), f[w], ldq(cpl + w * HXW + 4), dx[w]);
+        // first differences along y of the rows gy - 4 .. gy + 5: ey[i] between rows gy + i - 4 and gy + i - 3
+        Quad ey[9];
+        {
+            Quad prev = ldq(cpl - 4 * HXW);
+#pragma unroll
+            for (int i = 0; i < 9; ++i) {
+                const int rr = i - 3;
+                const Quad next = rr == 0 ? f[0] : rr == 1 ? f[1] : ldq(cpl + rr * HXW);
+                ey[i] = next - prev;
+                prev = next;
+            }
         }
-        const float4 f = q[4];
-        if (MODE != ST_LAPLACIAN) {
-            const u64 h0 = fma2(pk(v.x, v.y), pk(f.x, f.y), o0), h1 = fma2(pk(v.z, v.w), pk(f.z, f.w), o1);
-            if (MODE == ST_HAMILTONIAN) {
-                o0 = h0;
-                o1 = h1;
-            } else if (MODE == ST_HAM_RESIDUAL) {
-                // r = Hx - theta x (hi and lo parts of theta), w0 = r / max(diag_t + V - lambda, 0.1)
-                o0 = fma2(pk(-th_lo, -th_lo), pk(f.x, f.y), fma2(pk(-th_hi, -th_hi), pk(f.x, f.y), h0));
-                o1 = fma2(pk(-th_lo, -th_lo), pk(f.z, f.w), fma2(pk(-th_hi, -th_hi), pk(f.z, f.w), h1));
-                if (ok) {
-                    const float w0 = lo_of(o0) / fmaxf(p.diag_t + v.x - lam, 0.1f);
-                    const float w1 = hi_of(o0) / fmaxf(p.diag_t + v.y - lam, 0.1f);
-                    const float w2 = lo_of(o1) / fmaxf(p.diag_t + v.z - lam, 0.1f);
-                    const float w3 = hi_of(o1) / fmaxf(p.diag_t + v.w - lam, 0.1f);
-                    *reinterpret_cast<float4*>(orow2 + s * plane) = make_float4(w0, e1 ? w1 : 0.f, e2 ? w2 : 0.f, e3 ? w3 : 0.f);
-                    if (drow) {  // the sweeps' factor, as the JACOBI mode computes it
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+#pragma unroll
+            for (int w = 0; w < ROWS; ++w) {
+                const Quad d = (ey[4 + w + j] - ey[3 + w - j]) + dx[w][j];
+                acc[w] = fmaq(j == 3 ? k.b3 : j == 2 ? k.b2 : j == 1 ? k.b1 : k.b0, d, acc[w]);
+            }
+        }
+        if (NSIDE > 0) cp_async_wait<SD - 1>();
+        const float4* sl = side + (s % SD) * NSIDE * ROWS * THREADS;
+#pragma unroll
+        for (int w = 0; w < ROWS; ++w) {
+            Quad o = fmaq(k.hi, acc[w], mulq(k.lo, acc[w]));
+            if (MODE != ST_LAPLACIAN && ok[w]) {
+                const float4 v = sl[w * THREADS];
+                const Quad h = fmaq(ldq(sl + w * THREADS), f[w], o);
+                if (MODE == ST_HAMILTONIAN) {
+                    o = h;
+                } else if (MODE == ST_HAM_RESIDUAL) {
+                    // r = Hx - theta x (hi and lo parts of theta), w0 = r / max(diag_t + V - lambda, 0.1)
+                    o = fmaq(rep(-th_lo), f[w], fmaq(rep(-th_hi), f[w], h));
+                    const float w0 = lo_of(o.a) / fmaxf(p.diag_t + v.x - lam, 0.1f);
+                    const float w1 = hi_of(o.a) / fmaxf(p.diag_t + v.y - lam, 0.1f);
+                    const float w2 = lo_of(o.b) / fmaxf(p.diag_t + v.z - lam, 0.1f);
+                    const float w3 = hi_of(o.b) / fmaxf(p.diag_t + v.w - lam, 0.1f);
+                    *reinterpret_cast<float4*>(obase2 + (off + w * p.P)) = make_float4(w0, e1 ? w1 : 0.f, e2 ? w2 : 0.f, e3 ? w3 : 0.f);
+                    if (dbase) {  // the sweeps' factor, as the JACOBI mode computes it
                         const float d0 = p.omega * (1.0f / fmaxf(p.diag_t + v.x - lam, 0.1f));
                         const float d1 = p.omega * (1.0f / fmaxf(p.diag_t + v.y - lam, 0.1f));
                         const float d2 = p.omega * (1.0f / fmaxf(p.diag_t + v.z - lam, 0.1f));
                         const float d3 = p.omega * (1.0f / fmaxf(p.diag_t + v.w - lam, 0.1f));
-                        *reinterpret_cast<float4*>(drow + s * plane) = make_float4(d0, e1 ? d1 : 0.f, e2 ? d2 : 0.f, e3 ? d3 : 0.f);
+                        *reinterpret_cast<float4*>(dbase + (off + w * p.P)) = make_float4(d0, e1 ? d1 : 0.f, e2 ? d2 : 0.f, e3 ? d3 : 0.f);
                     }
-                }
-            } else {
-                const u64 nl = pk(-lam, -lam);
-                // w + (omega / max(diag_t + V - lambda, 0.1)) (r - (H w - lambda w)), as the scalar sweep (an
-                // approximate division measured 2 % faster per solve but moved the NH3 96^3 finite-difference check of
-                // the adjoint past its bound: the sweep keeps the IEEE division)
-                const u64 u0 = sub2(pk(r.x, r.y), fma2(nl, pk(f.x, f.y), h0));
-                const u64 u1 = sub2(pk(r.z, r.w), fma2(nl, pk(f.z, f.w), h1));
-                float i0, i1, i2, i3;
-                if (drow) {  // the factor stored by the residual pass of this iteration
-                    i0 = dq.x;
-                    i1 = dq.y;
-                    i2 = dq.z;
-                    i3 = dq.w;
                 } else {
-                    i0 = p.omega * (1.0f / fmaxf(p.diag_t + v.x - lam, 0.1f));
-                    i1 = p.omega * (1.0f / fmaxf(p.diag_t + v.y - lam, 0.1f));
-                    i2 = p.omega * (1.0f / fmaxf(p.diag_t + v.z - lam, 0.1f));
-                    i3 = p.omega * (1.0f / fmaxf(p.diag_t + v.w - lam, 0.1f));
+                    // w + (omega / max(diag_t + V - lambda, 0.1)) (r - (H w - lambda w)), as the scalar sweep (an
+                    // approximate division measured 2 % faster per solve but moved the NH3 96^3 finite-difference check
+                    // of the adjoint past its bound: the sweep keeps the IEEE division)
+                    const Quad u = ldq(sl + (ROWS + w) * THREADS) - fmaq(rep(-lam), f[w], h);
+                    Quad fac;
+                    if (dbase) {  // the factor stored by the residual pass of this iteration
+                        fac = ldq(sl + (2 * ROWS + w) * THREADS);
+                    } else {
+                        fac.a = pk(p.omega * (1.0f / fmaxf(p.diag_t + v.x - lam, 0.1f)), p.omega * (1.0f / fmaxf(p.diag_t + v.y - lam, 0.1f)));
+                        fac.b = pk(p.omega * (1.0f / fmaxf(p.diag_t + v.z - lam, 0.1f)), p.omega * (1.0f / fmaxf(p.diag_t + v.w - lam, 0.1f)));
+                    }
+                    o = fmaq(fac, u, f[w]);
                 }
-                o0 = fma2(pk(i0, i1), u0, pk(f.x, f.y));
-                o1 = fma2(pk(i2, i3), u1, pk(f.z, f.w));
             }
-        }
-        if (ok) {
-            *reinterpret_cast<float4*>(orow + s * plane) =
-                make_float4(lo_of(o0), e1 ? hi_of(o0) : 0.f, e2 ? lo_of(o1) : 0.f, e3 ? hi_of(o1) : 0.f);
-            if (DOT) {
-                if (MODE == ST_HAM_RESIDUAL) {
-                    const double r0 = lo_of(o0), r1 = hi_of(o0), r2 = lo_of(o1), r3 = hi_of(o1);
-                    dot += r0 * r0;
-                    if (e1) dot += r1 * r1;
-                    if (e2) dot += r2 * r2;
-                    if (e3) dot += r3 * r3;
-                } else {
-                    dot += quad_dot(f, o0, o1, e1, e2, e3);
-                }
+            if (ok[w]) {
+                store_quad(obase + (off + w * p.P), o, e1, e2, e3);
+                if (DOT) dot += quad_dot(MODE == ST_HAM_RESIDUAL ? o : f[w], o, e1, e2, e3);
             }
         }
         __syncthreads();  // the centre plane's buffer is free
-        if (alive && threadIdx.x == 0 && s + 12 < nplanes) {
-            issue(s + 12);
-            issued = s + 13;
+        if (alive && threadIdx.x == 0 && s + 4 + NS < nplanes) {
+            proxy_fence();
+            issue(s + 4 + NS);
+            issued = s + 5 + NS;
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = q[i + 1];  // the z-queue moves up one plane
+        if (++sn == NS) { sn = 0; pn ^= 1u; }
+        if (++sc == NS) sc = 0;
     }
     // after a wait gave up: the latest copy issued into each slot may still be in flight (a parity wait on a slot's
     // latest copy is unambiguous, and returns at once for one that arrived)
@@ -419,20 +479,52 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 struct Shape { int tiles_x, tiles_y, chunks, zc; };
 
+// The tile width of an n^3 grid: the fewest tile columns for the work in them. A tile's plane costs its arithmetic, which
+// grows with the width, but no less than a fixed part (the 24 TMA rows, the barrier), about that of 42 columns: a row of tiles
+// costs tiles x max(264, 6.25 BX). Measured per launch with every width forced to 32 / 48 / 64 (us): the sweep at 48^3 k = 4
+// 10.9 / 10.7 / 10.7 and H at k = 8 12.9 / 10.7 / 12.7; 64^3 k = 8 16.2 / 18.9 / 14.8; 95^3 k = 8 31.2 / 29.1 / 36.7; 128^3
+// k = 20 147 / 158 / 125; H at 128^3 k = 40 177 / 197 / 176.
+int tile_width(int n) {
+    int best = 32;
+    double cost = 1e30;
+    for (int bx : {32, 48, 64}) {
+        const double c = ceil_div(n, bx) * std::max(264.0, 6.25 * bx);
+        if (c < cost) {
+            cost = c;
+            best = bx;
+        }
+    }
+    return best;
+}
+
+// shared memory of a launch, and the CTAs of it that an SM holds: 228 KB with 1 KB reserved per CTA, of which the
+// kernel's static part is under 1 KB
+template <int MODE, int BX>
+constexpr int smem_bytes() { return ring_depth<MODE>() * (int)Tile<BX>::PLANE_BYTES + SD * n_side<MODE>() * ROWS * Tile<BX>::THREADS * 16; }
+template <int MODE, int BX>
+constexpr int ctas_of() {
+    const int by_smem = (228 * 1024) / (smem_bytes<MODE, BX>() + 1536);
+    return by_smem < Tile<BX>::CTAS_PER_SM ? by_smem : Tile<BX>::CTAS_PER_SM;
+}
+int ctas_per_sm(int mode, int bx) {
+    if (mode == ST_JACOBI) return bx == 32 ? ctas_of<ST_JACOBI, 32>() : bx == 48 ? ctas_of<ST_JACOBI, 48>() : ctas_of<ST_JACOBI, 64>();
+    return bx == 32 ? ctas_of<ST_HAMILTONIAN, 32>() : bx == 48 ? ctas_of<ST_HAMILTONIAN, 48>() : ctas_of<ST_HAMILTONIAN, 64>();
+}
+
 // The grid: (x, y) tiles x vectors x z-chunks. A CTA's time is about (its planes + prologue) steps
-// whatever else runs (the kernel is latency-bound at CTAS_PER_SM CTAs per SM), and the launch takes
-// ceil(CTAs / resident slots) such rounds, so the chunk count minimises waves x (zc + c) with c the
-// fixed cost of a chunk in plane steps (its 8 halo planes, partly hidden behind the other resident
-// CTAs; c = 8 measured best against 12 and 4). At 95^3 with 5 CTAs per SM this gives 5 chunks of 19
-// planes for 8 and 16 vectors (720 and 1440 CTAs) and 3 chunks of 32 planes for 48 and 64 vectors.
-Shape shape_for(const Layout& L, int count) {
+// whatever else runs, and the launch takes ceil(CTAs / resident slots) such rounds, so the chunk count minimises
+// waves x (zc + c) with c the fixed cost of a chunk in plane steps (its 8 halo planes, partly hidden behind the other
+// resident CTAs; c = 8 measured best against 12 and 4). Chunks go down to 4 planes, which only grids that leave the chip
+// idle reach (33^3 x 3: 6.2 us against 8.3 us with chunks of 8).
+Shape shape_for(const Layout& L, int count, int mode) {
+    const int bx = tile_width(L.n);
     Shape sh;
-    sh.tiles_x = ceil_div(L.n, BX);
+    sh.tiles_x = ceil_div(L.n, bx);
     sh.tiles_y = ceil_div(L.n, BY);
     const long long per_chunk = (long long)sh.tiles_x * sh.tiles_y * count;
-    const long long slots = (long long)CTAS_PER_SM * sm_count();
+    const long long slots = (long long)ctas_per_sm(mode, bx) * sm_count();
     long long best = -1;
-    for (int c = 1; c <= std::max(1, L.n / 8); ++c) {
+    for (int c = 1; c <= std::max(1, L.n / 4); ++c) {
         const int zc = ceil_div(L.n, c);
         const int cc = ceil_div(L.n, zc);
         const long long waves = (cc * per_chunk + slots - 1) / slots;
@@ -449,7 +541,7 @@ Shape shape_for(const Layout& L, int count) {
 // the shape of a launch with c z-chunks per tile column
 Shape shape_with_chunks(const Layout& L, int c) {
     Shape sh;
-    sh.tiles_x = ceil_div(L.n, BX);
+    sh.tiles_x = ceil_div(L.n, tile_width(L.n));
     sh.tiles_y = ceil_div(L.n, BY);
     sh.zc = ceil_div(L.n, std::max(1, std::min(c, L.n)));
     sh.chunks = ceil_div(L.n, sh.zc);
@@ -469,18 +561,26 @@ int current_device() {
     return d;
 }
 
-template <int MODE, bool DOT>
-void launch_mode(const Shape& sh, int count, const CUtensorMap& tmap, const Params& p, float* out, cudaStream_t s) {
-    const int smem = NS * PLANE_BYTES + SD * n_side<MODE>() * THREADS * 16;
+template <int MODE, bool DOT, int BX>
+void launch_tile(const Shape& sh, int count, const CUtensorMap& tmap, const Params& p, float* out, cudaStream_t s) {
+    constexpr int smem = smem_bytes<MODE, BX>();
     static std::atomic<unsigned long long> attr_set{0};
-    once_per_device(attr_set, [smem] {
-        KS_CUDA(cudaFuncSetAttribute(stencil_kernel<MODE, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        // CTAS_PER_SM rings of 30 KB need the large shared-memory carveout
-        KS_CUDA(cudaFuncSetAttribute(stencil_kernel<MODE, DOT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    once_per_device(attr_set, [] {
+        KS_CUDA(cudaFuncSetAttribute(stencil_kernel<MODE, DOT, BX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        // the rings of an SM's CTAs need the large shared-memory carveout
+        KS_CUDA(cudaFuncSetAttribute(stencil_kernel<MODE, DOT, BX>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     });
     dim3 grid(sh.tiles_x * sh.tiles_y * sh.chunks, count);
-    stencil_kernel<MODE, DOT><<<grid, THREADS, smem, s>>>(tmap, p, out);
+    stencil_kernel<MODE, DOT, BX><<<grid, Tile<BX>::THREADS, smem, s>>>(tmap, p, out);
     KS_LAUNCH_CHECK();
+}
+
+template <int MODE, bool DOT>
+void launch_mode(const Shape& sh, int count, const CUtensorMap& tmap, const Params& p, float* out, cudaStream_t s) {
+    const int bx = tile_width(p.n);
+    if (bx == 32) launch_tile<MODE, DOT, 32>(sh, count, tmap, p, out, s);
+    else if (bx == 48) launch_tile<MODE, DOT, 48>(sh, count, tmap, p, out, s);
+    else launch_tile<MODE, DOT, 64>(sh, count, tmap, p, out, s);
 }
 
 }  // namespace
@@ -488,7 +588,7 @@ void launch_mode(const Shape& sh, int count, const CUtensorMap& tmap, const Para
 void make_field_tmap(CUtensorMap* map, const Layout& L, const float* base, int count) {
     cuuint64_t dims[4] = {(cuuint64_t)L.n, (cuuint64_t)L.n, (cuuint64_t)L.n, (cuuint64_t)count};
     cuuint64_t strides[3] = {(cuuint64_t)L.P * 4, (cuuint64_t)L.n * L.P * 4, (cuuint64_t)L.F * 4};
-    cuuint32_t box[4] = {HXW, HYW, 1, 1};
+    cuuint32_t box[4] = {(cuuint32_t)(tile_width(L.n) + 8), HYW, 1, 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides, box, estr,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -514,7 +614,7 @@ int stencil_tuned_chunks(int n, int count, int mode) {
 
 int stencil_max_chunks(const Layout& L) { return std::max(1, L.n / 8); }
 
-int stencil_model_chunks(const Layout& L, int count) { return shape_for(L, count).chunks; }
+int stencil_model_chunks(const Layout& L, int count) { return shape_for(L, count, ST_HAMILTONIAN).chunks; }
 
 std::vector<std::array<int, 4>> stencil_tuning_entries() {
     const int dev = current_device();
@@ -534,12 +634,12 @@ void stencil_tuning_clear() {
 }
 
 int stencil_ctas(const Layout& L, int count) {
-    Shape sh = shape_for(L, count);
+    Shape sh = shape_for(L, count, ST_HAMILTONIAN);
     return sh.tiles_x * sh.tiles_y * sh.chunks * count;
 }
 
 int stencil_ctas_per_vector(const Layout& L, int count) {
-    Shape sh = shape_for(L, count);
+    Shape sh = shape_for(L, count, ST_HAM_RESIDUAL);
     return sh.tiles_x * sh.tiles_y * sh.chunks;
 }
 
@@ -555,7 +655,7 @@ int launch_stencil(const Layout& L, const CUtensorMap& tmap, int count, const St
     int chunks = a.chunks;
     if (chunks <= 0 && !dot && (a.mode == ST_HAMILTONIAN || a.mode == ST_JACOBI)) chunks = stencil_tuned_chunks(L.n, count, a.mode);
     if (chunks > 0 && dot) throw std::invalid_argument("stencil: a forced chunking is for the launches without dot partials");
-    Shape sh = chunks > 0 ? shape_with_chunks(L, chunks) : shape_for(L, count);
+    Shape sh = chunks > 0 ? shape_with_chunks(L, chunks) : shape_for(L, count, a.mode);
     Params p;
     p.n = L.n;
     p.P = L.P;
@@ -563,7 +663,9 @@ int launch_stencil(const Layout& L, const CUtensorMap& tmap, int count, const St
     p.tiles_x = sh.tiles_x;
     p.tiles_y = sh.tiles_y;
     p.zc = sh.zc;
-    p.scale = a.scale;
+    const double scale = a.scale * KAPPA;
+    p.scale_hi = (float)scale;
+    p.scale_lo = (float)(scale - (double)p.scale_hi);
     p.omega = a.omega;
     p.diag_t = a.diag_t;
     p.V = a.V;

@@ -72,7 +72,7 @@ void launch_scale_ratio(long long F, float* x, const double* sum_dev, double tar
 enum StencilMode { ST_LAPLACIAN = 0, ST_HAMILTONIAN = 1, ST_JACOBI = 2, ST_HAM_RESIDUAL = 3 };
 struct StencilArgs {
     int mode = ST_LAPLACIAN;
-    float scale = 0;        // multiplies sum_m c_m (second differences): 1/h^2 or -1/(2 h^2)
+    double scale = 0;       // multiplies sum_m c_m (second differences): 1/h^2 or -1/(2 h^2)
     const float* V = nullptr;   // potential (HAMILTONIAN, JACOBI)
     const float* R = nullptr;   // JACOBI right-hand sides (block, stride F)
     const double* lambda = nullptr; // JACOBI shift per vector (device)

@@ -576,7 +576,7 @@ void Poisson::iteration(float* v, int par) {
     double* scal = scal_.d();
     StencilArgs lapd;
     lapd.mode = ST_LAPLACIAN;
-    lapd.scale = (float)(1.0 / (L_.h * L_.h));
+    lapd.scale = 1.0 / (L_.h * L_.h);
     lapd.dot_partials = red_->partials();
     const int ctas = launch_stencil(L_, p_.tmap, 1, lapd, ap_.at(0), s_);
     launch_finish(red_->partials(), ctas, 1, -1.0, scal, s_);
@@ -648,7 +648,7 @@ void Poisson::moments(const float* rho, double* dst) {
 void Poisson::true_residual(const CUtensorMap& v_map) {
     StencilArgs a;
     a.mode = ST_LAPLACIAN;
-    a.scale = (float)(1.0 / (L_.h * L_.h));
+    a.scale = 1.0 / (L_.h * L_.h);
     launch_stencil(L_, v_map, 1, a, ap_.at(0), s_);
     Terms t;
     t.count = 2;
@@ -668,7 +668,7 @@ PoissonStats Poisson::solve(const float* rho, float* v, const CUtensorMap& v_map
     // r = b - A v = b + L v; z = M^-1 r; p = z
     StencilArgs lap;
     lap.mode = ST_LAPLACIAN;
-    lap.scale = (float)(1.0 / (L_.h * L_.h));
+    lap.scale = 1.0 / (L_.h * L_.h);
     launch_stencil(L_, v_map, 1, lap, ap_.at(0), s_);
     Terms t;
     t.count = 2;
@@ -931,7 +931,7 @@ EigenStats Solver::lobpcg(Channel& ch, Lane& lane, const float* V, double tol, d
     const int rb0 = lane.red.readbacks;
     const double omega = jacobi_omega();
     const double diag_t = -1.5 * COEFF0 / (L_.h * L_.h);
-    const float ham_scale = (float)(-0.5 / (L_.h * L_.h));
+    const double ham_scale = -0.5 / (L_.h * L_.h);
     double* theta_d = ch.theta_d.d();
     double* lambda_d = theta_d + k;
     double* coef_d = theta_d + 2 * k;
@@ -1892,7 +1892,7 @@ ks_status Solver::solve(const ks_nucleus* nuc, int nn, int n_up, int n_dn, const
             const int cols = fd ? kk[sp] : nocc[sp];
             StencilArgs kin;
             kin.mode = ST_LAPLACIAN;
-            kin.scale = (float)(-0.5 / (L_.h * L_.h));
+            kin.scale = -0.5 / (L_.h * L_.h);
             launch_stencil(L_, ch_[sp].A[ch_[sp].cur].tmap, cols, kin, ch_[sp].T.at(0), s_);
             for (int i = 0; i < cols; ++i) {
                 pairs.push_back({ch_[sp].A[ch_[sp].cur].at(i), ch_[sp].T.at(i)});

@@ -55,3 +55,32 @@ def test_gram_pieces_match_f64(ks, n, m, mt, gram_mode):
     assert err < (2e-6 if gram_mode == 1 and (m > 32 or mt > 32) else 20 * U), err
     if gram_mode == 0:
         assert np.array_equal(g[:, :m], g[:, :m].T)
+
+
+@pytest.mark.parametrize("n", [31, 47, 49, 63, 64, 65, 95, 97])
+def test_stencil_tile_widths(ks, oracle, n):
+    """H psi, the Laplacian and the sweeps just below, at and above the tile widths 32, 48 and 64 and their multiples, for
+    one vector and for five, and with every z-chunking (down to one plane per chunk) the same bits. Bounds as the
+    kernels' other tests: each output is 24 products of neighbouring differences, 1e-6 of the largest term in f32."""
+    h, lam = 0.27, -0.4
+    x, y, z = oracle.grid_points(n, h)
+    rng = np.random.default_rng(n)
+    v = f32(-2 * np.exp(-(x * x + y * y + z * z)))
+    psi = f32(np.stack([np.exp(-((x - c) ** 2 + y * y + z * z) / 3) + 1e-3 * rng.uniform(-1, 1, n ** 3) for c in (0.0, 0.4, -0.3, 0.7, 0.2)]))
+    try:
+        ks.clear_stencil_tuning()
+        gpu = ks.apply_hamiltonian(n, h, psi, v)
+        for i in (0, 4):
+            want = oracle.hamiltonian(n, h, psi[i], v)
+            assert np.abs(gpu[i] - want).max() < 1e-6 * (np.abs(want).max() + np.abs(v * psi[i]).max())
+        one = ks.apply_hamiltonian(n, h, psi[:1], v)
+        assert np.array_equal(one[0], gpu[0])
+        for chunks in (1, 2, 7, n // 4, n):
+            ks.set_stencil_tuning([(n, 1, 1, chunks)])
+            assert np.array_equal(ks.apply_hamiltonian(n, h, psi[:1], v), one), chunks
+    finally:
+        ks.clear_stencil_tuning()
+    lap = oracle.laplacian(n, h, psi[1])
+    assert np.abs(ks.apply_laplacian(n, h, psi[1]) - lap).max() < 1e-6 * np.abs(lap).max()
+    want = oracle.jacobi_precond(n, h, v, lam, psi[2])
+    assert np.abs(ks.apply_precond(n, h, v, lam, psi[2]) - want).max() < 2e-6 * np.abs(want).max()
