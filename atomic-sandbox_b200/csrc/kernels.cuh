@@ -172,25 +172,28 @@ void launch_forces(const Layout& L, const float* rho, const Nuc* nuc, int nn, do
 void launch_poisson_rhs(const Layout& L, const float* rho, const double* q, double* ghost, float* b, cudaStream_t s);
 // multigrid level descriptor: Dirichlet boundary d_low/d_high spacings beyond the first/last point
 struct MgLevel { int n, P; long long F; double h; float g_low, g_high; };
-void launch_mg_jacobi(const MgLevel& lv, const float* x, const float* b, float* out, float omega, cudaStream_t s);
+void launch_mg_first(const MgLevel& lv, const float* b, float* x, float omega, cudaStream_t s);  // two sweeps from x = 0
+// out = one sweep on x (out != x); partials (or null): [mg_sweep_ctas][2] of b.out and b.b
+void launch_mg_sweep(const MgLevel& lv, const float* x, const float* b, float* out, float omega, double* partials, cudaStream_t s);
+int mg_sweep_ctas(const MgLevel& lv);
 void launch_mg_residual(const MgLevel& lv, const float* x, const float* b, float* out, cudaStream_t s);
-void launch_mg_restrict(const MgLevel& coarse, const MgLevel& fine, const float* rf, float* bc, cudaStream_t s);
-void launch_mg_prolong_add(const MgLevel& coarse, const MgLevel& fine, const float* xc, float* xf, cudaStream_t s);
-// all levels from `first` to the coarsest in one single-CTA launch (levels small enough for one SM)
+void launch_mg_restrict(const MgLevel& coarse, const MgLevel& fine, const float* r, float* bc, cudaStream_t s);
+void launch_mg_prolong_add(const MgLevel& coarse, const MgLevel& fine, const float* xc, float* x, cudaStream_t s);
+// the levels of at most MG_COARSE_N points per axis in one single-CTA launch: lv[0]'s right-hand side b, solution x
+constexpr int MG_COARSE_N = 12;
 struct MgCoarse {
     static constexpr int MAXL = 8;
     int nlev = 0;
     MgLevel lv[MAXL];
-    float* x[MAXL];
-    float* b[MAXL];
-    float* res[MAXL];
-    float* tmp[MAXL];
 };
-void launch_mg_coarse(const MgCoarse& c, float omega, int pre, int post, int coarsest_sweeps, cudaStream_t s);
-// CG updates with the scalars read on the device (scal: f64 solver scalars; scal[0] = p.Ap,
-// scal[rz_slot] = r.z): v += alpha p, r += alpha (L p) with alpha = r.z / p.Ap (A = -L); and
-// p = z + beta p with beta = scal[rz_new] / scal[rz_old]. A non-positive p.Ap or r.z gives alpha = 0.
-void launch_cg_update(long long F, float* v, float* r, const float* p, const float* ap, const double* scal, int rz_slot, cudaStream_t s);
-void launch_cg_direction(long long F, float* p, const float* z, const double* scal, int rz_old, int rz_new, cudaStream_t s);
+void launch_mg_coarse(const MgCoarse& c, const float* b, float* x, float omega, int coarsest_sweeps, cudaStream_t s);
+// CG updates with the scalars on the device (scal: f64 solver scalars; scal[rz_slot] = r.z): v += alpha p, r += alpha (L p) with
+// alpha = r.z / p.Ap (A = -L), p.Ap minus the sum of the `count` partials (written to pap_out); and p = z + beta p with
+// beta = r.z / scal[rz_old], r.z and r.r the sums of the `count` partial pairs (written to scal[rz_new], scal[rz_new + 1] and
+// dots_out; rz_old < 0: p = z). A non-positive p.Ap or r.z gives alpha = 0.
+void launch_cg_update(long long F, float* v, float* r, const float* p, const float* ap, const double* partials, int count, const double* scal,
+                      int rz_slot, double* pap_out, cudaStream_t s);
+void launch_cg_direction(long long F, float* p, const float* z, const double* partials, int count, double* scal, int rz_old, int rz_new,
+                         double* dots_out, cudaStream_t s);
 
 }  // namespace ks

@@ -128,9 +128,8 @@ constexpr double LAST_STEP_RESIDUAL_FACTOR = 3.0;
 constexpr double BOUNDARY_DENSITY_WARN = 1e-5;
 constexpr double STALL_LEVEL_PER_ELECTRON = 1e-3;
 // multigrid (crates/qm-gpu/src/multigrid.rs:62-72)
-constexpr int PRE_SWEEPS = 2, POST_SWEEPS = 2, COARSEST_SWEEPS = 12;
+constexpr int COARSEST_SWEEPS = 12;  // two sweeps before and two after on every other level
 constexpr double MG_OMEGA = 6.0 / 7.0;
-constexpr int FUSED_MAX_N = 12;
 constexpr int CHECK_EVERY = 5;
 
 double jacobi_omega() {
@@ -497,7 +496,7 @@ void Poisson::init(const Layout& L, cudaStream_t s, Reducer* red) {
     L_ = L;
     s_ = s;
     red_ = red;
-    r_.create(L, 1); p_.create(L, 1); ap_.create(L, 1); b_.create(L, 1); z_.create(L, 1); res0_.create(L, 1); tmp0_.create(L, 1);
+    r_.create(L, 1); p_.create(L, 1); ap_.create(L, 1); b_.create(L, 1); z_.create(L, 1); tmp0_.create(L, 1);
     ghost_.alloc(24 * (size_t)L.n * L.n * sizeof(double));
     scal_.alloc(8 * sizeof(double));
     zero_device(scal_.p, 8 * sizeof(double));
@@ -520,55 +519,62 @@ void Poisson::init(const Layout& L, cudaStream_t s, Reducer* red) {
         d_low = dl;
         d_high = dh;
     }
-    levels_.resize(lvdesc_.size());
-    for (size_t l = 1; l < lvdesc_.size(); ++l) {
-        size_t bytes = (size_t)lvdesc_[l].F * sizeof(float);
-        levels_[l].lv = lvdesc_[l];
-        levels_[l].x.alloc(bytes); levels_[l].b.alloc(bytes); levels_[l].res.alloc(bytes); levels_[l].tmp.alloc(bytes);
-        zero_device(levels_[l].x.p, bytes); zero_device(levels_[l].b.p, bytes);
-        zero_device(levels_[l].res.p, bytes); zero_device(levels_[l].tmp.p, bytes);
-    }
     fused_from_ = (int)lvdesc_.size() - 1;
     for (size_t l = 0; l < lvdesc_.size(); ++l)
-        if (lvdesc_[l].n <= FUSED_MAX_N) { fused_from_ = (int)l; break; }
+        if (lvdesc_[l].n <= MG_COARSE_N) { fused_from_ = (int)l; break; }
+    levels_.resize(fused_from_ + 1);  // the deeper levels live in the coarse kernel's shared memory
+    for (int l = 1; l <= fused_from_; ++l) {
+        size_t bytes = (size_t)lvdesc_[l].F * sizeof(float);
+        levels_[l].lv = lvdesc_[l];
+        levels_[l].x.alloc(bytes); levels_[l].b.alloc(bytes); levels_[l].tmp.alloc(bytes);
+        zero_device(levels_[l].x.p, bytes); zero_device(levels_[l].b.p, bytes); zero_device(levels_[l].tmp.p, bytes);
+    }
+    zpart_.alloc(2 * (size_t)std::max(mg_sweep_ctas(lvdesc_[0]), red_->blocks()) * sizeof(double));
 }
 
-void Poisson::cycle(int l, float* x, const float* b) {
+void Poisson::cycle(int l, float* x, const float* b, double* partials) {
     const int nl = (int)lvdesc_.size();
-    auto res_of = [&](int i) { return i == 0 ? res0_.at(0) : levels_[i].res.f(); };
-    auto tmp_of = [&](int i) { return i == 0 ? tmp0_.at(0) : levels_[i].tmp.f(); };
     if (l >= fused_from_) {
         MgCoarse c;
         c.nlev = nl - l;
         if (c.nlev > MgCoarse::MAXL) throw std::logic_error("multigrid: too many fused levels");
-        for (int i = l; i < nl; ++i) {
-            int q = i - l;
-            c.lv[q] = lvdesc_[i];
-            c.x[q] = i == l ? x : levels_[i].x.f();
-            c.b[q] = i == l ? const_cast<float*>(b) : levels_[i].b.f();
-            c.res[q] = res_of(i);
-            c.tmp[q] = tmp_of(i);
-        }
-        launch_mg_coarse(c, (float)MG_OMEGA, PRE_SWEEPS, POST_SWEEPS, COARSEST_SWEEPS, s_);
+        for (int i = l; i < nl; ++i) c.lv[i - l] = lvdesc_[i];
+        launch_mg_coarse(c, b, x, (float)MG_OMEGA, COARSEST_SWEEPS, s_);
         return;
     }
+    // two sweeps each way (crates/qm-gpu/src/multigrid.rs:62-72); the residual passes through the level's scratch
     const MgLevel& lv = lvdesc_[l];
-    launch_fill(x, 0.0f, lv.F, s_);
-    for (int sw = 0; sw < PRE_SWEEPS; ++sw) {
-        if (sw & 1) launch_mg_jacobi(lv, tmp_of(l), b, x, (float)MG_OMEGA, s_);
-        else launch_mg_jacobi(lv, x, b, tmp_of(l), (float)MG_OMEGA, s_);
-    }
-    launch_mg_residual(lv, x, b, res_of(l), s_);
-    launch_mg_restrict(lvdesc_[l + 1], lv, res_of(l), levels_[l + 1].b.f(), s_);
-    cycle(l + 1, levels_[l + 1].x.f(), levels_[l + 1].b.f());
+    float* tmp = l == 0 ? tmp0_.at(0) : levels_[l].tmp.f();
+    launch_mg_first(lv, b, x, (float)MG_OMEGA, s_);
+    launch_mg_residual(lv, x, b, tmp, s_);
+    launch_mg_restrict(lvdesc_[l + 1], lv, tmp, levels_[l + 1].b.f(), s_);
+    cycle(l + 1, levels_[l + 1].x.f(), levels_[l + 1].b.f(), nullptr);
     launch_mg_prolong_add(lvdesc_[l + 1], lv, levels_[l + 1].x.f(), x, s_);
-    for (int sw = 0; sw < POST_SWEEPS; ++sw) {
-        if (sw & 1) launch_mg_jacobi(lv, tmp_of(l), b, x, (float)MG_OMEGA, s_);
-        else launch_mg_jacobi(lv, x, b, tmp_of(l), (float)MG_OMEGA, s_);
-    }
+    launch_mg_sweep(lv, x, b, tmp, (float)MG_OMEGA, nullptr, s_);
+    launch_mg_sweep(lv, tmp, b, x, (float)MG_OMEGA, partials, s_);
 }
 
-void Poisson::vcycle(const float* rhs, float* z) { cycle(0, z, rhs); }
+int Poisson::vcycle(const float* rhs, float* z) {
+    int count;
+    if (fused_from_ == 0) {  // the whole cycle in one CTA: the dot products are a launch of their own
+        cycle(0, z, rhs, nullptr);
+        Pairs p;
+        p.count = 2;
+        p.a[0] = rhs; p.b[0] = z;
+        p.a[1] = rhs; p.b[1] = rhs;
+        count = red_->blocks();
+        launch_dots(L_.F, p, zpart_.d(), count, s_);
+    } else {
+        cycle(0, z, rhs, zpart_.d());
+        count = mg_sweep_ctas(lvdesc_[0]);
+    }
+    if (count > 2048) {  // every CTA of the next kernel sums the pairs: beyond 32 KB a launch of its own is cheaper
+        launch_finish(zpart_.d(), count, 2, 1.0, red_->res() + 8, s_);
+        KS_CUDA(cudaMemcpyAsync(zpart_.p, red_->res() + 8, 2 * sizeof(double), cudaMemcpyDeviceToDevice, s_));
+        count = 1;
+    }
+    return count;
+}
 
 // One PCG iteration between two readbacks (crates/qm-gpu/src/poisson.rs:284-342): ap = L p with p.Ap, the v / r update,
 // z = M^-1 r by one V-cycle, r.z and r.r, the new direction. The scalars stay on the device (parity par).
@@ -579,17 +585,13 @@ void Poisson::iteration(float* v, int par) {
     lapd.scale = 1.0 / (L_.h * L_.h);
     lapd.dot_partials = red_->partials();
     const int ctas = launch_stencil(L_, p_.tmap, 1, lapd, ap_.at(0), s_);
-    launch_finish(red_->partials(), ctas, 1, -1.0, scal, s_);
-    launch_cg_update(L_.F, v, r_.at(0), p_.at(0), ap_.at(0), scal, 1 + 2 * par, s_);
-    vcycle(r_.at(0), z_.at(0));
-    const int nxt = 1 - par;
-    red_->dots({{r_.at(0), z_.at(0)}, {r_.at(0), r_.at(0)}}, 1, 1.0);
-    KS_CUDA(cudaMemcpyAsync(scal + 1 + 2 * nxt, red_->res() + 1, 2 * sizeof(double), cudaMemcpyDeviceToDevice, s_));
-    launch_cg_direction(L_.F, p_.at(0), z_.at(0), scal, 1 + 2 * par, 1 + 2 * nxt, s_);
-    KS_CUDA(cudaMemcpyAsync(red_->res(), scal, sizeof(double), cudaMemcpyDeviceToDevice, s_));
+    // res[0] = p.Ap, res[1], res[2] = r.z, r.r: what the host reads after the iteration
+    launch_cg_update(L_.F, v, r_.at(0), p_.at(0), ap_.at(0), red_->partials(), ctas, scal, 1 + 2 * par, red_->res(), s_);
+    const int count = vcycle(r_.at(0), z_.at(0));
+    launch_cg_direction(L_.F, p_.at(0), z_.at(0), zpart_.d(), count, scal, 1 + 2 * par, 1 + 2 * (1 - par), red_->res() + 1, s_);
 }
 
-// The iteration's ~40 small launches (the V-cycle's coarse levels are a few microseconds each) replayed as one CUDA
+// The iteration's small launches (a few microseconds each) replayed as one CUDA
 // graph per (v, parity): captured on first use, then one cudaGraphLaunch per iteration, so the device runs them
 // back to back instead of waiting on the host's launch rate. The graph's kernels count as launches at every replay.
 void Poisson::run_iteration(float* v, int par) {
@@ -675,14 +677,10 @@ PoissonStats Poisson::solve(const float* rho, float* v, const CUtensorMap& v_map
     t.x[0] = b_.at(0); t.c[0] = 1.f;
     t.x[1] = ap_.at(0); t.c[1] = 1.f;
     launch_lincomb(L_.F, 1, r_.at(0), t, s_);
-    vcycle(r_.at(0), z_.at(0));
-    Terms cp;
-    cp.count = 1;
-    cp.x[0] = z_.at(0); cp.c[0] = 1.f;
-    launch_lincomb(L_.F, 1, p_.at(0), cp, s_);
+    const int count = vcycle(r_.at(0), z_.at(0));
+    red_->dots({{b_.at(0), b_.at(0)}}, 2, 1.0);
     // scal[1 + 2s] = r.z, scal[2 + 2s] = r.r for parity s
-    red_->dots({{r_.at(0), z_.at(0)}, {r_.at(0), r_.at(0)}, {b_.at(0), b_.at(0)}}, 0, 1.0);
-    KS_CUDA(cudaMemcpyAsync(scal + 1, red_->res(), 2 * sizeof(double), cudaMemcpyDeviceToDevice, s_));
+    launch_cg_direction(L_.F, p_.at(0), z_.at(0), zpart_.d(), count, scal, -1, 1, red_->res(), s_);
     const double* h = red_->read(3);
     const double bb = h[2];
     double rz = h[0], rr = h[1];
@@ -800,10 +798,10 @@ size_t Solver::footprint_bytes(int n, int n_up, int n_dn, const SolverOptions& o
     size_t total = 0;
     total += 11 * rounded(field);                                        // potentials, densities, XC, ones
     total += 3 * (rounded(((size_t)1 << 20) * sizeof(double)) + rounded(Reducer::RES_CAP * sizeof(double)));  // reducers
-    total += 7 * rounded(field) + rounded(24 * (size_t)n * n * sizeof(double));  // Poisson CG fields and ghost table
-    for (int m = n; m > 2;) {                                            // multigrid levels, four fields each
+    total += 6 * rounded(field) + rounded(24 * (size_t)n * n * sizeof(double));  // Poisson CG fields and ghost table
+    for (int m = n; m > MG_COARSE_N;) {                                  // multigrid levels, three fields each
         m /= 2;
-        total += 4 * rounded((size_t)Layout::make(m, 1.0).F * sizeof(float));
+        total += 3 * rounded((size_t)Layout::make(m, 1.0).F * sizeof(float));
     }
     for (int ne : {n_up, n_dn}) {
         if (ne <= 0) continue;

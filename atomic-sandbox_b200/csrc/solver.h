@@ -192,9 +192,10 @@ public:
     void moments(const float* rho, double* dst_dev);  // 49 f64, dV applied
 
 private:
-    struct Level { MgLevel lv; DevBuf x, b, res, tmp; };
-    void vcycle(const float* rhs, float* z);
-    void cycle(int l, float* x, const float* b);
+    struct Level { MgLevel lv; DevBuf x, b, tmp; };
+    // z = M^-1 rhs by one V-cycle; leaves the partial pairs (rhs.z, rhs.rhs) in zpart_ and returns their count
+    int vcycle(const float* rhs, float* z);
+    void cycle(int l, float* x, const float* b, double* partials);
     void true_residual(const CUtensorMap& v_map);  // r = b + L v into ap_, |r|^2 reduced (v is v_map's field)
     void iteration(float* v, int par);
     void run_iteration(float* v, int par);
@@ -205,9 +206,10 @@ private:
     Layout L_;
     cudaStream_t s_ = nullptr;
     Reducer* red_ = nullptr;
-    Block r_, p_, ap_, b_, z_, res0_, tmp0_;
+    Block r_, p_, ap_, b_, z_, tmp0_;
     DevBuf ghost_, scal_, q_;
-    std::vector<Level> levels_;   // coarse levels 1..; level 0 is the fine grid (its x/b are z/r)
+    DevBuf zpart_;                // per-CTA pairs (r.z, r.r) of the V-cycle's last kernel
+    std::vector<Level> levels_;   // coarse levels 1..fused_from_; level 0 is the fine grid (its x/b are z/r)
     int fused_from_ = 0;          // first level handled by the single-CTA kernel
     std::vector<MgLevel> lvdesc_;
 };

@@ -84,3 +84,19 @@ def test_stencil_tile_widths(ks, oracle, n):
     assert np.abs(ks.apply_laplacian(n, h, psi[1]) - lap).max() < 1e-6 * np.abs(lap).max()
     want = oracle.jacobi_precond(n, h, v, lam, psi[2])
     assert np.abs(ks.apply_precond(n, h, v, lam, psi[2]) - want).max() < 2e-6 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n", [5, 11, 12, 13, 24, 25, 26, 33, 52])
+def test_poisson_level_edges(ks, oracle, n):
+    """The Hartree solve where its multigrid levels change: the whole cycle in one CTA (n <= 12), one level above it (13,
+    24, 25), two (26, 33, 52), even and odd sizes. Against the f64 solve, with the f32 floor of the single-grid test
+    (2e-5 for a potential of order 1), and in no more iterations than a working V-cycle takes (unpreconditioned
+    CG on 26^3 takes above 60)."""
+    h = 12.0 / n
+    x, y, z = oracle.grid_points(n, h)
+    s = max(0.8, h)
+    rho = (2 * np.pi * s * s) ** -1.5 * np.exp(-((x - 0.5) ** 2 + (y + 0.3) ** 2 + z * z) / (2 * s * s))
+    v, it, res = ks.poisson_solve(n, h, rho, tol=1e-7)
+    vo, _, _ = oracle.poisson_solve(n, h, f32(rho), tol=1e-11)
+    assert it <= 40, it
+    assert np.abs(v - vo).max() < 2e-5 * max(1.0, np.abs(vo).max()), (it, res)
