@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(GW * 32) gram_kernel(long long F, int m, const
 // redundant are skipped, and with LOWER also those of S^T T above the diagonal, which a Rayleigh-Ritz step never reads
 // (24 patches instead of 30).
 // Measured (with the finish): m = mt = 24 on 95^3 99.7 -> 57.3 us, 8 / 8 69 -> 24.6, 128^3 24 / 24 208 -> 114, 48^3 12 / 12 25.8 ->
-// 16.4; in a solve, where LOWER applies, 96.7 -> 49.6 us. Bound by the FMA pipe's packed instructions (math_pipe_throttle is
-// the top stall, one per four cycles and scheduler) at 3.3 TB/s. Scalar FMAs took the same time. Rows of 512 bytes by one bulk
+// 16.4; in a solve, where LOWER applies, 96.7 -> 49.6 us. At 3.3 TB/s it is bound by the FMA pipe
+// (58 % active, math_pipe_throttle first) and fixed latencies at 12 to 16 warps per SM. Scalar FMAs took the same time. Rows of 512 bytes by one bulk
 // copy each, at a padded pitch, measured slower: 85 us copied by the consumers, 95 us by a producer warp.
 // Sums: f32 over 16 points of a slab, f32 over a warp's slabs, f64 across the warps and (launch_finish) the CTAs.
 // Larger blocks are several pieces: DIAG pieces (rows, the same columns of S and of T) and pieces of one foreign column block.
@@ -223,18 +223,19 @@ constexpr int g_warps() {
     int n = 0;
     for (int i = 0; i < 2 * M8; ++i)
         for (int j = 0; j < (DIAG ? M8 : 0) + T8; ++j) n += g_patch<M8, DIAG, LOWER>(i, j);
-    // 128, 168 or 255 registers each; two slots of 7 KB and more do not fit for 16 warps
-    return n <= 24 && M8 + T8 <= 6 ? 16 : n <= 32 ? 12 : 8;
+    // 128, 168 or 255 registers each; two slots of 7 KB (9 KB) and more do not fit for 16 (12) warps
+    return n <= 24 && M8 + T8 <= 6 ? 16 : n <= 32 && M8 + T8 <= 8 ? 12 : 8;
 }
 
 // Rows: fields [32 rb, 32 rb + 8 M8) of S. DIAG: columns the same fields of S, then fields [32 rb, 32 rb + 8 T8) of T. Else
-// the columns are the fields [32 cb, 32 cb + 8 T8) of tm_t's block (nt fields), at column colT of G. mc: columns of G.
+// the columns are the fields [CB cb, CB cb + 8 T8) of tm_t's block (nt fields), at column colT of G. mc: columns of G.
 template <int M8, int T8, bool DIAG, bool LOWER, int DEPTH>
 __global__ void __launch_bounds__(32 * g_warps<M8, T8, DIAG, LOWER>(), 1)
     gram_piece_kernel(const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_t, int slabs, int m, int nt, int mc,
                       int rb, int cb, int colT, bool mirrorT, double* __restrict__ partials, int* err) {
     constexpr int W = g_warps<M8, T8, DIAG, LOWER>();
     constexpr int RI = 2 * M8, C = (DIAG ? M8 : 0) + T8, SLAB = (M8 + T8) * 1024;
+    constexpr int CB = T8 > 4 ? 64 : 32;  // column blocks
     extern __shared__ unsigned char g_raw[];
     unsigned char* base = g_raw + ((1024 - (g_su32(g_raw) & 1023)) & 1023);
     __shared__ __align__(8) uint64_t full[W * DEPTH];
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(32 * g_warps<M8, T8, DIAG, LOWER>(), 1)
         unsigned char* dst = mine + (size_t)d * SLAB;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(g_su32(&bars[d])), "r"((unsigned)SLAB) : "memory");
         g_tma(dst, &tm_s, x, 32 * rb, &bars[d]);  // whole boxes land, the zero fill past F and past the last field included
-        if (T8 > 0) g_tma(dst + M8 * 1024, &tm_t, x, 32 * tb, &bars[d]);
+        if (T8 > 0) g_tma(dst + M8 * 1024, &tm_t, x, CB * tb, &bars[d]);
     };
     int issued = min(DEPTH, nmine);
     if (lane == 0)
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(32 * g_warps<M8, T8, DIAG, LOWER>(), 1)
                 if (col != row) out[(size_t)col * mc + row] = v;
             }
         } else {
-            const int t = 32 * (DIAG ? rb : cb) + b + 8 * (j - (DIAG ? M8 : 0));
+            const int t = CB * (DIAG ? rb : cb) + b + 8 * (j - (DIAG ? M8 : 0));
             if (t < nt) {
                 out[(size_t)row * mc + colT + t] = v;
                 if (mirrorT) out[(size_t)t * mc + row] = v;  // a foreign block of S itself: both halves of S^T S
@@ -404,14 +405,15 @@ void launch_gram_diag(int m8, int t8, bool lower, int blocks, long long F, const
     }
 #define KS_GRAM_DIAGS(M) KS_GRAM_DIAG(M, 0) KS_GRAM_DIAG(M, 1) KS_GRAM_DIAG(M, 2) KS_GRAM_DIAG(M, 3) KS_GRAM_DIAG(M, 4)
     KS_GRAM_DIAGS(1) KS_GRAM_DIAGS(2) KS_GRAM_DIAGS(3) KS_GRAM_DIAGS(4)
+    KS_GRAM_DIAG(1, 5) KS_GRAM_DIAG(1, 6) KS_GRAM_DIAG(1, 7) KS_GRAM_DIAG(1, 8)
 #undef KS_GRAM_DIAGS
 #undef KS_GRAM_DIAG
     throw std::logic_error("gram: piece out of range");
 }
 
-// a piece of m8 row groups and the 32 fields of T from 32 cb on
+// a piece of m8 row groups and column block cb of T: 64 fields for one row group, else 32
 void launch_gram_foreign(int m8, int blocks, long long F, const GramMaps& g, int m, int mt, int rb, int cb, double* partials, cudaStream_t s) {
-    if (m8 == 1) launch_gram_piece<1, 4, false, false>(blocks, F, g.s, g.t, m, mt, m + mt, rb, cb, m, false, partials, s);
+    if (m8 == 1) launch_gram_piece<1, 8, false, false>(blocks, F, g.s, g.t, m, mt, m + mt, rb, cb, m, false, partials, s);
     else if (m8 == 2) launch_gram_piece<2, 4, false, false>(blocks, F, g.s, g.t, m, mt, m + mt, rb, cb, m, false, partials, s);
     else if (m8 == 3) launch_gram_piece<3, 4, false, false>(blocks, F, g.s, g.t, m, mt, m + mt, rb, cb, m, false, partials, s);
     else launch_gram_piece<4, 4, false, false>(blocks, F, g.s, g.t, m, mt, m + mt, rb, cb, m, false, partials, s);
@@ -660,11 +662,12 @@ int launch_gram(long long F, int m, const float* S, int mt, const float* T, doub
         KS_LAUNCH_CHECK();
         return blocks;
     }
-    // 32 x 32 pieces, the row groups of 8 exact where there is one row block (m = 8, mt = 120 on 48^3 with 32-row pieces
-    // took 53 us instead of 33): per row block the DIAG piece with its own T block (if there is one), then the foreign blocks of S below
-    // the diagonal (mirrored) and the other blocks of T
-    const int nr = ceil_div(m, 32), nt = ceil_div(mt, 32);
-    const int m8 = nr == 1 ? ceil_div(m, 8) : 4, t8 = nt > 1 ? 4 : ceil_div(mt, 8);
+    // 32 x 32 pieces, the row groups of 8 exact where there is one row block, and 64 columns of T for one row group, whose
+    // pieces repeat the most (m = 8, mt = 120 on 48^3 / 95^3: with 8 x 32 33 / 136 us, with 8 x 64 23 / 119 us): per row
+    // block the DIAG piece with its own T block (if there is one), then the foreign blocks of S below the diagonal
+    // (mirrored) and the other blocks of T
+    const int cw = m <= 8 ? 64 : 32, nr = ceil_div(m, 32), nt = ceil_div(mt, cw);
+    const int m8 = nr == 1 ? ceil_div(m, 8) : 4, t8 = nt > 1 ? cw / 8 : ceil_div(mt, 8);
     GramMaps g;
     g_rows_map(&g.s, S, F, m, 8 * m8);
     if (mt > 0) g_rows_map(&g.t, T, F, mt, 8 * (nr > 1 ? 4 : t8));

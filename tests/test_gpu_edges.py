@@ -36,7 +36,7 @@ def test_block_update_over_solves(ks, oracle, n, k):
         assert np.sqrt((r * r).sum() / (xs[i] * xs[i]).sum()) < tol * max(1.0, abs(ev[i])) + 63 * U * hnorm, (i, it)
 
 
-@pytest.mark.parametrize("n,m,mt", [(5, 1, 1), (9, 8, 8), (17, 9, 7), (29, 24, 24), (25, 17, 32), (33, 32, 32), (13, 33, 1), (13, 8, 33), (29, 8, 120),
+@pytest.mark.parametrize("n,m,mt", [(5, 1, 1), (9, 8, 8), (17, 9, 7), (29, 24, 24), (25, 17, 32), (33, 32, 32), (13, 33, 1), (13, 8, 33), (9, 5, 64), (13, 7, 65), (29, 8, 120),
                                     (25, 12, 40), (25, 20, 60), (17, 40, 8), (21, 60, 60), (33, 33, 33)])
 @pytest.mark.parametrize("gram_mode", [0, 1])
 def test_gram_pieces_match_f64(ks, n, m, mt, gram_mode):
