@@ -17,9 +17,11 @@
 // seven outputs it belongs to (ZRow), so nothing moves between registers. The V / R reads (cp.async copies one plane ahead
 // into a small shared ring) and the stores are coalesced 16-byte accesses; the quad's pad columns are stored as 0.
 //
-// What bounds it: instruction issue. With one row per thread, a nine-deep register queue in z and symmetric differences
-// (the form this replaces) 128 outputs took 230 warp instructions, 32 of them register moves. Measured per launch, before and after: H psi on 95^3 x 16 vectors 43.0 -> 34.9 us,
-// on 128^3 x 40 216 -> 170 us, on 48^3 x 8 8.3 -> 7.2 us, a sweep on 128^3 x 20 in a solve 160 -> 125 us.
+// What bounds it: instruction issue and the fixed latencies behind it at 12 warps per SM (58 % of the issue slots, FMA pipe
+// 53 % active). With one row per thread, a nine-deep register queue in z and symmetric differences (the form this
+// replaces) 128 outputs took 250 warp instructions, now 173. Measured per launch, before and after: H psi on 95^3 x 16
+// vectors 43.0 -> 34.9 us, on 128^3 x 40 216 -> 170 us, on 48^3 x 8 8.3 -> 7.2 us, a sweep on 128^3 x 20 in a solve
+// 160 -> 125 us.
 #include <algorithm>
 #include <map>
 #include <mutex>
