@@ -158,8 +158,9 @@ __global__ void lincomb_kernel(long long n4, float4* __restrict__ y, Terms t) {
 // not stored: a test per output inside the loop kept its shared loads from being issued ahead. Bound by the shared loads
 // of the inputs (once per group of QG outputs) beside HBM. One CTA per slice and group of 16 outputs (the form this
 // replaces) read every input once per group from L2 and had no copy behind its arithmetic: m = 60, q = 40 on 128^3
-// 858 -> 253 us per launch (of 128 us for the bytes), m = 24, q = 16 on 95^3 37.0 -> 32.6 us. Two groups of 16 outputs
-// per thread measured slower (registers), 2 and 4 sets no faster than 3.
+// 858 -> 258 us per launch in a solve (of 128 us for the bytes), m = 24, q = 16 on 95^3 37.0 -> 36.1 us. Groups of 16 or 20
+// outputs on half the threads measured slower (373 and 312 us), 2 and 4 sets no faster than 3. The four components of one
+// output pair are consecutive: alternating between two pairs took 266 us.
 constexpr int QG = 8;
 constexpr int LCB = 64;          // float4 per field per stage: 1 KB copies
 constexpr int LC_RING = 16;      // stages at most
@@ -269,10 +270,9 @@ __global__ void __launch_bounds__(LC_THREADS + 32, 1) block_lincomb_kernel(long 
             for (int p4 = 0; p4 < QG / 4; ++p4) {
                 const ulonglong2 c4 = cs4[i * (QG / 4) + p4];  // (c_4p4, c_4p4+1), (c_4p4+2, c_4p4+3)
 #pragma unroll
-                for (int k2 = 0; k2 < 4; ++k2) {
-                    acc[2 * p4][k2] = lc_fma2(c4.x, vv[k2], acc[2 * p4][k2]);
-                    acc[2 * p4 + 1][k2] = lc_fma2(c4.y, vv[k2], acc[2 * p4 + 1][k2]);
-                }
+                for (int k2 = 0; k2 < 4; ++k2) acc[2 * p4][k2] = lc_fma2(c4.x, vv[k2], acc[2 * p4][k2]);
+#pragma unroll
+                for (int k2 = 0; k2 < 4; ++k2) acc[2 * p4 + 1][k2] = lc_fma2(c4.y, vv[k2], acc[2 * p4 + 1][k2]);
             }
         }
         // these reads of the slot come before the writes of the copies that refill it, which are the async proxy's
