@@ -8,12 +8,70 @@
 #include <algorithm>
 #include <cmath>
 
+// The O(n^3) loops run over contiguous elements whose sums do not depend on one another (never a dot product's own chain),
+// so the compiler vectorises them; with 4-wide AVX2 where the host has it. AVX2 without FMA: every element sees the same
+// roundings as the scalar loops, on every host.
+#if defined(__x86_64__) && defined(__GNUC__)
+#define KS_SIMD __attribute__((target_clones("avx2", "default")))
+#else
+#define KS_SIMD
+#endif
+
 namespace ks {
 namespace dense {
 
 namespace {
 constexpr double SYM_EIGEN_CHECK = 1e-11;  // crates/qm/src/eigen.rs:171
 }
+
+KS_SIMD void axpy(int n, double a, const double* __restrict__ x, double* __restrict__ y) {
+    for (int i = 0; i < n; ++i) y[i] += a * x[i];
+}
+
+namespace {
+// One QL sweep's rotations i = m - 1 .. l of the columns (i, i + 1) of Z, (z_i, z_i+1) <- (c_i z_i - s_i z_i+1,
+// s_i z_i + c_i z_i+1), for 8 rows of Z at a time: the column that two rotations share stays in registers.
+KS_SIMD void rotations(int n, int l, int m, const double* __restrict__ c, const double* __restrict__ s, double* __restrict__ z) {
+    int k = 0;
+    for (; k + 8 <= n; k += 8) {
+        double y[8];
+        for (int t = 0; t < 8; ++t) y[t] = z[(size_t)m * n + k + t];
+        for (int i = m - 1; i >= l; --i) {
+            double* zi = z + (size_t)i * n + k;
+            double* zn = zi + n;
+            for (int t = 0; t < 8; ++t) {
+                const double x = zi[t];
+                zn[t] = s[i] * x + c[i] * y[t];
+                y[t] = c[i] * x - s[i] * y[t];
+            }
+        }
+        for (int t = 0; t < 8; ++t) z[(size_t)l * n + k + t] = y[t];
+    }
+    for (; k < n; ++k) {
+        double y = z[(size_t)m * n + k];
+        for (int i = m - 1; i >= l; --i) {
+            const double x = z[(size_t)i * n + k];
+            z[(size_t)(i + 1) * n + k] = s[i] * x + c[i] * y;
+            y = c[i] * x - s[i] * y;
+        }
+        z[(size_t)l * n + k] = y;
+    }
+}
+// sqrt(a^2 + b^2) on the QL sweep's serial chain: in x87 extended precision nothing overflows or underflows and the one
+// rounding that counts is the last, at half of std::hypot's time
+double length(double a, double b) {
+#if defined(__x86_64__)
+    const long double x = a, y = b;
+    return (double)sqrtl(x * x + y * y);
+#else
+    return std::hypot(a, b);
+#endif
+}
+// a -= u x + v y
+KS_SIMD void rank2_row(int n, double u, const double* __restrict__ x, double v, const double* __restrict__ y, double* __restrict__ a) {
+    for (int i = 0; i < n; ++i) a[i] -= x[i] * u + y[i] * v;
+}
+}  // namespace
 
 void jacobi_eigen(int n, Mat a, std::vector<double>& evals, std::vector<double>& evecs) {
     auto A = [&](int i, int j) -> double& { return a[(size_t)i * n + j]; };
@@ -65,49 +123,48 @@ void tridiag_ql_eigen(int n, const Mat& a_in, std::vector<double>& evals, std::v
     evals.assign(n, 0.0);
     evecs.assign((size_t)n * n, 0.0);
     if (n == 0) return;
-    Mat A = a_in;
-    auto a = [&](int i, int j) -> double& { return A[(size_t)i * n + j]; };
-    Mat Z((size_t)n * n, 0.0);  // row-major accumulator, Z[r][c]
-    auto z = [&](int i, int j) -> double& { return Z[(size_t)i * n + j]; };
-    for (int i = 0; i < n; ++i) z(i, i) = 1.0;
+    // both work arrays transposed (column k of A at At + k n, of Z at Zt + k n), so that the loops below run along them
+    Mat At((size_t)n * n), Zt((size_t)n * n, 0.0);
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j) At[(size_t)j * n + i] = a_in[(size_t)i * n + j];
+    auto acol = [&](int j) { return At.data() + (size_t)j * n; };
+    auto zcol = [&](int j) { return Zt.data() + (size_t)j * n; };
+    for (int i = 0; i < n; ++i) zcol(i)[i] = 1.0;
     std::vector<double> v(n), p(n), w(n);
     // --- Householder: A <- H A H for k = 0..n-3, Z <- Z H
     for (int k = 0; k + 2 < n; ++k) {
+        const double* ak = acol(k);
         double tail = 0.0;
-        for (int i = k + 2; i < n; ++i) tail += a(i, k) * a(i, k);
+        for (int i = k + 2; i < n; ++i) tail += ak[i] * ak[i];
         if (tail == 0.0) continue;  // column already tridiagonal
-        double x0 = a(k + 1, k);
+        double x0 = ak[k + 1];
         double xnorm = std::sqrt(tail + x0 * x0);
         double alpha = x0 >= 0.0 ? -xnorm : xnorm;
         std::fill(v.begin(), v.end(), 0.0);
-        for (int i = k + 1; i < n; ++i) v[i] = a(i, k);
+        for (int i = k + 1; i < n; ++i) v[i] = ak[i];
         v[k + 1] -= alpha;
         double vn2 = 0.0;
         for (int i = k + 1; i < n; ++i) vn2 += v[i] * v[i];
         if (vn2 == 0.0) continue;
         double beta = 2.0 / vn2;
-        for (int i = k; i < n; ++i) {
-            double s = 0.0;
-            for (int j = k + 1; j < n; ++j) s += a(i, j) * v[j];
-            p[i] = beta * s;
-        }
+        std::fill(p.begin() + k, p.end(), 0.0);
+        for (int j = k + 1; j < n; ++j) axpy(n - k, v[j], acol(j) + k, p.data() + k);
+        for (int i = k; i < n; ++i) p[i] = beta * p[i];
         double K = 0.0;
         for (int j = k + 1; j < n; ++j) K += v[j] * p[j];
         K *= 0.5 * beta;
         for (int i = k; i < n; ++i) w[i] = p[i] - K * v[i];
         w[k] = p[k];  // v[k] = 0
-        for (int i = k; i < n; ++i)
-            for (int j = k; j < n; ++j) a(i, j) -= v[i] * w[j] + w[i] * v[j];
-        for (int r = 0; r < n; ++r) {
-            double qv = 0.0;
-            for (int j = k + 1; j < n; ++j) qv += z(r, j) * v[j];
-            qv *= beta;
-            for (int j = k + 1; j < n; ++j) z(r, j) -= qv * v[j];
-        }
+        for (int j = k; j < n; ++j) rank2_row(n - k, w[j], v.data() + k, v[j], w.data() + k, acol(j) + k);
+        // qv = beta Z v, Z -= qv v^T
+        std::fill(p.begin(), p.end(), 0.0);
+        for (int j = k + 1; j < n; ++j) axpy(n, v[j], zcol(j), p.data());
+        for (int r = 0; r < n; ++r) p[r] *= beta;
+        for (int j = k + 1; j < n; ++j) axpy(n, -v[j], p.data(), zcol(j));
     }
-    std::vector<double> d(n), e(n, 0.0);
-    for (int i = 0; i < n; ++i) d[i] = a(i, i);
-    for (int i = 0; i + 1 < n; ++i) e[i] = a(i + 1, i);
+    std::vector<double> d(n), e(n, 0.0), cs(n), sn(n);
+    for (int i = 0; i < n; ++i) d[i] = acol(i)[i];
+    for (int i = 0; i + 1 < n; ++i) e[i] = acol(i)[i + 1];
     // --- implicit QL with shifts on the tridiagonal (d, e), rotations accumulated into Z
     double f = 0.0, tst1 = 0.0;
     const double eps = std::ldexp(1.0, -52);
@@ -137,18 +194,16 @@ void tridiag_ql_eigen(int n, const Mat& a_in, std::vector<double>& evals, std::v
                     s2 = s;
                     g = c * e[i];
                     h = c * pp;
-                    r = std::hypot(pp, e[i]);
+                    r = length(pp, e[i]);
                     e[i + 1] = s * r;
                     s = e[i] / r;
                     c = pp / r;
                     pp = c * d[i] - s * g;
                     d[i + 1] = h + s * (c * g + s * d[i]);
-                    for (int k = 0; k < n; ++k) {
-                        double hz = z(k, i + 1);
-                        z(k, i + 1) = s * z(k, i) + c * hz;
-                        z(k, i) = c * z(k, i) - s * hz;
-                    }
+                    cs[i] = c;
+                    sn[i] = s;
                 }
+                rotations(n, l, m, cs.data(), sn.data(), Zt.data());
                 pp = -s * s2 * c3 * el1 * e[l] / dl1;
                 e[l] = s * pp;
                 d[l] = c * pp;
@@ -159,7 +214,7 @@ void tridiag_ql_eigen(int n, const Mat& a_in, std::vector<double>& evals, std::v
     }
     for (int k = 0; k < n; ++k) {
         evals[k] = d[k];
-        for (int i = 0; i < n; ++i) evecs[i + (size_t)n * k] = z(i, k);
+        std::copy(zcol(k), zcol(k) + n, evecs.begin() + (size_t)n * k);
     }
 }
 
@@ -168,13 +223,16 @@ void sym_eigen(int n, const Mat& a, std::vector<double>& evals, std::vector<doub
     double scale = 1.0;
     for (double l : evals) scale = std::max(scale, 1.0 + std::fabs(l));
     bool bad = false;
-    for (int k = 0; k < n && !bad; ++k) {
+    Mat at((size_t)n * n);
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j) at[(size_t)j * n + i] = a[(size_t)i * n + j];
+    std::vector<double> r(n);
+    for (int k = 0; k < n && !bad; ++k) {  // |A v - lambda v| of each pair
+        const double* v = evecs.data() + (size_t)n * k;
+        for (int i = 0; i < n; ++i) r[i] = -evals[k] * v[i];
+        for (int j = 0; j < n; ++j) axpy(n, v[j], at.data() + (size_t)j * n, r.data());
         double r2 = 0.0;
-        for (int i = 0; i < n; ++i) {
-            double s = -evals[k] * evecs[i + (size_t)n * k];
-            for (int j = 0; j < n; ++j) s += a[(size_t)i * n + j] * evecs[j + (size_t)n * k];
-            r2 += s * s;
-        }
+        for (int i = 0; i < n; ++i) r2 += r[i] * r[i];
         if (!(std::sqrt(r2) <= SYM_EIGEN_CHECK * scale)) bad = true;
     }
     if (!bad) return;
@@ -239,17 +297,15 @@ bool cholesky(int n, Mat& a) {
 }
 
 void cholesky_solve(int n, const Mat& l, int q, std::vector<double>& b) {
-    for (int c = 0; c < q; ++c) {
-        for (int i = 0; i < n; ++i) {
-            double s = b[(size_t)i * q + c];
-            for (int k = 0; k < i; ++k) s -= l[(size_t)i * n + k] * b[(size_t)k * q + c];
-            b[(size_t)i * q + c] = s / l[(size_t)i * n + i];
-        }
-        for (int i = n - 1; i >= 0; --i) {
-            double s = b[(size_t)i * q + c];
-            for (int k = i + 1; k < n; ++k) s -= l[(size_t)k * n + i] * b[(size_t)k * q + c];
-            b[(size_t)i * q + c] = s / l[(size_t)i * n + i];
-        }
+    // all right-hand sides together, row by row
+    auto row = [&](int i) { return b.data() + (size_t)i * q; };
+    for (int i = 0; i < n; ++i) {
+        for (int k = 0; k < i; ++k) axpy(q, -l[(size_t)i * n + k], row(k), row(i));
+        for (int c = 0; c < q; ++c) row(i)[c] /= l[(size_t)i * n + i];
+    }
+    for (int i = n - 1; i >= 0; --i) {
+        for (int k = i + 1; k < n; ++k) axpy(q, -l[(size_t)k * n + i], row(k), row(i));
+        for (int c = 0; c < q; ++c) row(i)[c] /= l[(size_t)i * n + i];
     }
 }
 

@@ -9,6 +9,9 @@ namespace dense {
 
 using Mat = std::vector<double>;  // row-major n x n
 
+// y += a x (vectorised over the elements: the same bits as a scalar loop)
+void axpy(int n, double a, const double* x, double* y);
+
 // Symmetric eigen-decomposition, checked like the reference's `qm::eigen::sym_eigen`
 // (crates/qm/src/eigen.rs:150-173): Householder tridiagonalisation + implicit QL, then every
 // pair's residual |A v - lambda v| against 1e-11 (1 + max|lambda|); a failing decomposition is

@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(32 * g_warps<M8, T8, DIAG, LOWER>(), 1)
     if (!alive && lane == 0)
         for (int k = max(0, issued - DEPTH); k < issued; ++k) g_wait(&bars[k % DEPTH], (unsigned)((k / DEPTH) & 1), 1LL << 16);
     __syncthreads();
-    // across the warps in f64, in warp order
+    // across the warps in f64, from the last warp to the first (the last ones hold the fewest slabs)
     float* red = reinterpret_cast<float*>(base);  // [warp][patch][lane]
 #pragma unroll
     for (int i = 0; i < RI; ++i)
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(32 * g_warps<M8, T8, DIAG, LOWER>(), 1)
         const int i = p / C, j = p % C;
         if (!g_patch<M8, DIAG, LOWER>(i, j)) continue;
         double v = 0.0;
-        for (int w = 0; w < W; ++w) v += (double)red[(w * RI * C + p) * 32 + lane];
+        for (int w = W - 1; w >= 0; --w) v += (double)red[(w * RI * C + p) * 32 + lane];
         const int row = 32 * rb + a + 4 * i;
         if (row >= m) continue;
         if (DIAG && j < M8) {

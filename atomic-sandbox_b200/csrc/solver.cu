@@ -203,23 +203,17 @@ double rayleigh_ritz(int m, const std::vector<double>& A, const std::vector<doub
     const int nkp = (int)keep.size();
     if (nkp < nk)
         throw NumericalError("lobpcg: the subspace lost rank (" + std::to_string(nkp) + " of " + std::to_string(m) + " kept)");
-    std::vector<double> T((size_t)m * nkp);  // m x nkp row-major
+    // T (m x nkp) row-major and its transpose; the products below run as axpys over contiguous rows, every element's
+    // sum in the index order of the plain triple loop
+    std::vector<double> T((size_t)m * nkp), Tt((size_t)m * nkp);
     for (int i = 0; i < m; ++i)
-        for (int c = 0; c < nkp; ++c) T[(size_t)i * nkp + c] = ub[i + (size_t)m * keep[c]] / std::sqrt(sb[keep[c]]);
+        for (int c = 0; c < nkp; ++c) Tt[(size_t)c * m + i] = T[(size_t)i * nkp + c] = ub[i + (size_t)m * keep[c]] / std::sqrt(sb[keep[c]]);
     std::vector<double> at((size_t)m * nkp, 0.0);  // an * T
     for (int i = 0; i < m; ++i)
-        for (int c = 0; c < nkp; ++c) {
-            double s = 0.0;
-            for (int j = 0; j < m; ++j) s += an[(size_t)i * m + j] * T[(size_t)j * nkp + c];
-            at[(size_t)i * nkp + c] = s;
-        }
-    dense::Mat ah((size_t)nkp * nkp);
-    for (int a = 0; a < nkp; ++a)
-        for (int b = 0; b < nkp; ++b) {
-            double s = 0.0;
-            for (int i = 0; i < m; ++i) s += T[(size_t)i * nkp + a] * at[(size_t)i * nkp + b];
-            ah[(size_t)a * nkp + b] = s;
-        }
+        for (int j = 0; j < m; ++j) dense::axpy(nkp, an[(size_t)i * m + j], &T[(size_t)j * nkp], &at[(size_t)i * nkp]);
+    dense::Mat ah((size_t)nkp * nkp, 0.0);
+    for (int i = 0; i < m; ++i)
+        for (int a = 0; a < nkp; ++a) dense::axpy(nkp, T[(size_t)i * nkp + a], &at[(size_t)i * nkp], &ah[(size_t)a * nkp]);
     for (int a = 0; a < nkp; ++a)
         for (int b = a + 1; b < nkp; ++b) {
             double s = 0.5 * (ah[(size_t)a * nkp + b] + ah[(size_t)b * nkp + a]);
@@ -242,12 +236,11 @@ double rayleigh_ritz(int m, const std::vector<double>& A, const std::vector<doub
         alpha = std::max(alpha, std::sqrt(s));
     }
     C.assign((size_t)m * nk, 0.0);  // column-major m x nk
-    for (int c = 0; c < nk; ++c)
-        for (int i = 0; i < m; ++i) {
-            double s = 0.0;
-            for (int q = 0; q < nkp; ++q) s += T[(size_t)i * nkp + q] * va[q + (size_t)nkp * order[c]];
-            C[i + (size_t)m * c] = d[i] * s;
-        }
+    for (int c = 0; c < nk; ++c) {
+        double* col = &C[(size_t)m * c];
+        for (int q = 0; q < nkp; ++q) dense::axpy(m, va[q + (size_t)nkp * order[c]], &Tt[(size_t)q * m], col);
+        for (int i = 0; i < m; ++i) col[i] = d[i] * col[i];
+    }
     return alpha;
 }
 
@@ -1172,12 +1165,12 @@ EigenStats Solver::lobpcg(Channel& ch, Lane& lane, const float* V, double tol, d
         for (int i = 0; i < k; ++i)
             for (int j = 0; j < k; ++j) bxx[(size_t)i * k + j] = B[(size_t)i * m + j];
         if (!dense::cholesky(k, bxx)) throw NumericalError("lobpcg: Cholesky of X^T X failed (X lost rank)");
-        for (int i = 0; i < k; ++i)
-            for (int c = 0; c < na_rr; ++c) {
-                double s = 0.0;
-                for (int j = 0; j < m; ++j) s += B[(size_t)i * m + j] * C[j + (size_t)m * c];
-                rhs[(size_t)i * na_rr + c] = s;
-            }
+        std::vector<double> xc(k);  // X^T B of one new column (B is symmetric: its rows are its columns)
+        for (int c = 0; c < na_rr; ++c) {
+            std::fill(xc.begin(), xc.end(), 0.0);
+            for (int j = 0; j < m; ++j) dense::axpy(k, C[j + (size_t)m * c], &B[(size_t)j * m], xc.data());
+            for (int i = 0; i < k; ++i) rhs[(size_t)i * na_rr + c] = xc[i];
+        }
         dense::cholesky_solve(k, bxx, na_rr, rhs);
         std::vector<double> coef((size_t)m * 2 * na_rr);
         for (int c = 0; c < na_rr; ++c)
