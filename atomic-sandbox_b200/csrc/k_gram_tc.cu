@@ -22,8 +22,9 @@
 // warp 13 lane 0 issues the hi*hi MMAs and warp 14 lane 0 the cross-term MMAs (the issue latency of
 // one thread, not the tensor core, is the limit), each committing to mbarriers; warps 0..7 drain
 // finished slots with tcgen05.ld (warp w: TMEM lane quadrant w % 4, column half w / 4), one row per
-// thread. The B operand is the A tile itself (its first N rows), so S is loaded once; every TMA
-// destination row is a multiple of 8, so 1024-byte aligned.
+// thread. The B operand is the A tile itself (its first N = round16(m) rows: at M = 128 the instruction
+// takes N in steps of 16), so S is loaded once; every TMA destination row is a multiple of 8, so
+// 1024-byte aligned. The rows of B past round8(m) are T rows and only make columns of D that nothing reads.
 //
 // The ring is what sets the speed: a stage's round trip (TMA, split, MMA, commit) takes a few
 // microseconds, so ~16 stages must be in flight per SM to stream at HBM rate. The tiles are
@@ -119,7 +120,9 @@ __device__ __forceinline__ float tf32_rn(float x) { return __uint_as_float((__fl
 struct Params {
     long long F;  // points per field (multiple of 4)
     int m, mt;
-    int TR0;      // first T row = MMA N: rows of the tile used as the B operand
+    int TR0;      // first T row, round8(m)
+    int N;        // MMA N: rows of the tile used as the B operand
+    unsigned idesc;  // instruction descriptor
     int rows;     // rows the split converts
     int stages_total;
     int R;        // ring depth
@@ -141,7 +144,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
     __shared__ unsigned tmem_base;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nbuf = min(NBUF_MAX, 512 / (2 * p.TR0));  // TMEM: nbuf buffers of two N-column slots (hi*hi, cross)
+    const int nbuf = min(NBUF_MAX, 512 / (2 * p.N));  // TMEM: nbuf buffers of two N-column slots (hi*hi, cross)
     // this CTA's contiguous range of stages (32 points each)
     const int per = (p.stages_total + gridDim.x - 1) / gridDim.x;
     const int s0 = blockIdx.x * per;
@@ -227,7 +230,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
         // whole-range cross-term slot biased the Gram by ~1e-7 relative). Descriptors advance by the
         // tile size (ring) and 32 B per K-step (the address field counts 16-byte units).
         if (lane == 0) {
-            const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(p.TR0 >> 3) << 17) | ((unsigned)(ROWS >> 4) << 24);
+            const unsigned idesc = p.idesc;
             const unsigned long long dh0 = smem_desc(su32(hi)), dl0 = smem_desc(su32(lo));
             const unsigned long long step = (unsigned long long)(p.tbytes >> 4);
             const bool main_issuer = warp == 13;
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
                 if (i >= nbuf && !mbar_wait(&acc_empty[b], bph ^ 1u, p.err)) break;
                 if (!mbar_wait(&conv[s], ph, p.err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned d = tmem + (unsigned)(2 * b * p.TR0) + (main_issuer ? 0u : (unsigned)p.TR0);
+                const unsigned d = tmem + (unsigned)(2 * b * p.N) + (main_issuer ? 0u : (unsigned)p.N);
                 const unsigned long long h0 = dh0 + (unsigned long long)s * step, l0 = dl0 + (unsigned long long)s * step;
                 if (main_issuer) {
                     mma_tf32(d, h0, h0, idesc, 0u);
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
         for (int i = 0; i < nst; ++i) {
             if (!mbar_wait(&acc_full[b], bph, p.err)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned ta = lane_base + (unsigned)(2 * b * p.TR0);
+            const unsigned ta = lane_base + (unsigned)(2 * b * p.N);
             // 16 columns of both slots per tcgen05.ld round (registers: the 64-column form has 32 per thread)
 #pragma unroll
             for (int g0 = 0; g0 < HALF; g0 += 16) {
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
                 for (int g = 0; g < 16; g += 8)
                     if (g0 + g < ncols) {
                         ld8(r + g, ta + g0 + g);
-                        ld8(rx + g, ta + p.TR0 + g0 + g);
+                        ld8(rx + g, ta + p.N + g0 + g);
                     }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -349,6 +352,13 @@ void make_rows_map(CUtensorMap* map, const float* base, long long F, int rows) {
 
 int gram_tc_blocks() { return sm_count(); }
 
+// tf32 operands, f32 accumulators, N / 8 in bits 17..22, M / 16 in bits 24..28. kind::tf32 with one CTA and M = 128 takes
+// N = 16, 32, .. 256 only; N = round16(m) <= round8(m) + 8 lies inside the tile, which holds at least 8 rows of T.
+unsigned gram_tc_idesc(int m) {
+    const unsigned N = (unsigned)((m + 15) & ~15);
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((N >> 3) << 17) | ((unsigned)(ROWS >> 4) << 24);
+}
+
 // Where the mixed form takes this kernel: blocks beyond one CUDA-core piece, which it then beats (m = mt = 60 on 128^3: 356 us
 // against 540 in pieces, in a solve). Within one piece the CUDA cores read every field once too, are limited by it and round
 // to nearest (m = mt = 24 on 95^3: 49.5 us against 74 here, with errors of 1e-8 against 2e-7).
@@ -367,6 +377,8 @@ void launch_gram_tc(long long F, int m, const float* S, int mt, const float* T, 
     p.mt = mt;
     const int m8 = (m + 7) & ~7, mt8 = (mt + 7) & ~7;
     p.TR0 = m8;
+    p.idesc = gram_tc_idesc(m);
+    p.N = (int)((p.idesc >> 17) & 63u) << 3;
     p.rows = m8 + mt8;
     p.tbytes = p.rows * KT * 4;
     p.stages_total = (int)((F + KT - 1) / KT);

@@ -126,6 +126,7 @@ void launch_finish_pair(const FinishDesc& a, const FinishDesc& b, cudaStream_t s
 // G = S^T [S | T] on the tensor cores (k_gram_tc.cu): partials [gram_tc_blocks()][(m + mt) x m] of the
 // transpose D = [S | T]^T S; m <= 64, round8(m) + mt <= 128.
 int gram_tc_blocks();
+unsigned gram_tc_idesc(int m);  // the MMA's instruction descriptor
 bool gram_tc_wins(int m, int mt);  // where the mixed form uses it: blocks beyond one CUDA-core piece
 void launch_gram_tc(long long F, int m, const float* S, int mt, const float* T, double* partials, cudaStream_t s);
 int reduce_blocks(long long F);

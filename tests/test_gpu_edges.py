@@ -100,3 +100,27 @@ def test_poisson_level_edges(ks, oracle, n):
     vo, _, _ = oracle.poisson_solve(n, h, f32(rho), tol=1e-11)
     assert it <= 40, it
     assert np.abs(v - vo).max() < 2e-5 * max(1.0, np.abs(vo).max()), (it, res)
+
+
+@pytest.mark.parametrize("n,m,mt", [(9, 1, 33), (13, 8, 40), (13, 9, 112), (13, 17, 64), (13, 24, 33), (21, 33, 33), (21, 40, 40), (21, 41, 41),
+                                    (21, 48, 48), (13, 49, 1), (13, 49, 72), (21, 56, 56), (21, 57, 57), (13, 64, 64)])
+def test_tensor_core_gram_shapes(ks, n, m, mt):
+    """Every class of N = round16(m) of the tensor-core form against round8(m), with T blocks up to the largest, one stage
+    per CTA and several. Bound: hi holds 11 bits, so the dropped lo lo term is below 2^-20 |s| |t|, the two rounded lo
+    operands add 2^-22 each, and the truncating sums of a stage's 12 products at most 12 ulp of 2^-24 between them:
+    together under 2e-6."""
+    rng = np.random.default_rng(100 * m + mt)
+    s, t = f32(rng.standard_normal((m, n ** 3))), f32(rng.standard_normal((mt, n ** 3)))
+    g = ks.gram(n, s, t, gram_mode=1)
+    st = np.concatenate([s, t])
+    scale = np.sqrt(np.outer((s * s).sum(1), (st * st).sum(1)))
+    err = (np.abs(g - s @ st.T) / scale).max()
+    assert err < 2e-6, err
+
+
+@pytest.mark.parametrize("m,mt", [(8, 8), (10, 15), (24, 24), (32, 32)])
+def test_mixed_form_of_small_blocks_is_the_plain_form(ks, m, mt):
+    """Up to 32 columns the mixed form takes the CUDA cores: the same bits as the plain form."""
+    rng = np.random.default_rng(m)
+    s, t = rng.standard_normal((m, 13 ** 3)), rng.standard_normal((mt, 13 ** 3))
+    assert np.array_equal(ks.gram(13, s, t, gram_mode=1), ks.gram(13, s, t, gram_mode=0))
