@@ -100,3 +100,19 @@ def test_autotuner_arguments_are_refused_before_any_device_work(ks):
         ks.set_stencil_tuning([(95, 8, 1, 96)])  # more chunks than planes
     with pytest.raises(ValueError):
         ks.set_stencil_tuning([(95, 0, 1, 5)])
+
+
+def test_hpsi_device_takes_addresses_only(ks):
+    """hpsi_device's pointers are device addresses: None is the null pointer (KS_INVALID before any device call), and
+    whatever is not an integer is refused, host buffers above all."""
+    good = [0, 33, 0.25, 3, 1 << 40, 1 << 41, 1 << 42]
+    for i in (4, 5, 6):
+        with pytest.raises(ValueError):
+            ks.hpsi_device(*[None if j == i else a for j, a in enumerate(good)])
+    for i in (0, 4, 5, 6):
+        for bad in ("psi", b"psi", 1.0, ctypes.c_void_p(1 << 40), (ctypes.c_float * 4)(), [1 << 40]):
+            with pytest.raises(TypeError):
+                ks.hpsi_device(*[bad if j == i else a for j, a in enumerate(good)])
+    for n, h, count in ((4, 0.25, 3), (1025, 0.25, 3), (33, 0.0, 3), (33, 0.25, 0)):
+        with pytest.raises(ValueError):
+            ks.hpsi_device(0, n, h, count, 1 << 40, 1 << 41, 1 << 42)
