@@ -748,12 +748,14 @@ ks_status ks_autotune_stencil(int n, const int* counts, int ncount, int* chunks_
                     a.diag_t = (float)(1.5 * 205.0 / 72.0 / (h * h));
                     a.dinv = d.at(0);
                 }
-                // every distinct chunking of the candidates 1 .. max: the best of three timings of four launches each
+                // the cost model's choice, then every other distinct chunking of the candidates 1 .. max: the best of three
+                // timings of four launches each
+                const int model_c = stencil_model_chunks(L, k, a.mode), model_zc = (n + model_c - 1) / model_c;
                 int best_c = 0, last_zc = -1;
                 float best_ms = 0.f;
-                for (int c = 1; c <= stencil_max_chunks(L); ++c) {
-                    const int zc = (n + c - 1) / c;
-                    if (zc == last_zc) continue;
+                for (int i_c = 0; i_c <= stencil_max_chunks(L); ++i_c) {
+                    const int c = i_c == 0 ? model_c : i_c, zc = (n + c - 1) / c;
+                    if (i_c > 0 && (zc == last_zc || zc == model_zc)) continue;
                     last_zc = zc;
                     a.chunks = c;
                     for (int w = 0; w < 2; ++w) launch_stencil(L, x.tmap, k, a, y.at(0), sc.s);

@@ -526,7 +526,7 @@ Shape shape_for(const Layout& L, int count, int mode) {
     const long long per_chunk = (long long)sh.tiles_x * sh.tiles_y * count;
     const long long slots = (long long)ctas_per_sm(mode, bx) * sm_count();
     long long best = -1;
-    for (int c = 1; c <= std::max(1, L.n / 4); ++c) {
+    for (int c = 1; c <= stencil_max_chunks(L); ++c) {
         const int zc = ceil_div(L.n, c);
         const int cc = ceil_div(L.n, zc);
         const long long waves = (cc * per_chunk + slots - 1) / slots;
@@ -614,9 +614,10 @@ int stencil_tuned_chunks(int n, int count, int mode) {
     return it == tune_table().end() ? 0 : it->second;
 }
 
-int stencil_max_chunks(const Layout& L) { return std::max(1, L.n / 8); }
+// chunks of 4 planes at least: what the cost model searches and the autotuner times
+int stencil_max_chunks(const Layout& L) { return std::max(1, L.n / 4); }
 
-int stencil_model_chunks(const Layout& L, int count) { return shape_for(L, count, ST_HAMILTONIAN).chunks; }
+int stencil_model_chunks(const Layout& L, int count, int mode) { return shape_for(L, count, mode).chunks; }
 
 std::vector<std::array<int, 4>> stencil_tuning_entries() {
     const int dev = current_device();
@@ -633,11 +634,6 @@ void stencil_tuning_clear() {
     for (auto it = tune_table().begin(); it != tune_table().end();)
         it = std::get<0>(it->first) == dev ? tune_table().erase(it) : std::next(it);
     tune_entries.store((int)tune_table().size());
-}
-
-int stencil_ctas(const Layout& L, int count) {
-    Shape sh = shape_for(L, count, ST_HAMILTONIAN);
-    return sh.tiles_x * sh.tiles_y * sh.chunks * count;
 }
 
 int stencil_ctas_per_vector(const Layout& L, int count) {

@@ -94,7 +94,7 @@ struct StencilArgs {
 void stencil_set_tuned_chunks(int n, int count, int mode, int chunks);
 int stencil_tuned_chunks(int n, int count, int mode);  // 0: none
 int stencil_max_chunks(const Layout& L);                // the candidates are 1 .. this
-int stencil_model_chunks(const Layout& L, int count);   // the cost model's choice
+int stencil_model_chunks(const Layout& L, int count, int mode);  // the cost model's choice, one of them
 // the current device's entries as (n, count, mode, chunks) quadruples
 std::vector<std::array<int, 4>> stencil_tuning_entries();
 void stencil_tuning_clear();
@@ -105,7 +105,6 @@ int stencil_ctas_per_vector(const Layout& L, int count);
 int launch_stencil(const Layout& L, const CUtensorMap& tmap, int count, const StencilArgs& a, float* out, cudaStream_t s);
 // A 4-D tensor map (n, n, n, count) over a block of pitched fields with the stencil's halo box.
 void make_field_tmap(CUtensorMap* map, const Layout& L, const float* base, int count);
-int stencil_ctas(const Layout& L, int count);
 
 // ---------------------------------------------------------------- reductions (k_reduce.cu)
 // Deterministic two-stage reductions: a kernel writes one f64 partial per CTA and value, then
