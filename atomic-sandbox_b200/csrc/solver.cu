@@ -547,7 +547,7 @@ void Poisson::cycle(int l, float* x, const float* b, double* partials) {
     launch_mg_sweep(lv, tmp, b, x, (float)MG_OMEGA, partials, s_);
 }
 
-int Poisson::vcycle(const float* rhs, float* z) {
+Poisson::Pairs2 Poisson::vcycle(const float* rhs, float* z) {
     int count;
     if (fused_from_ == 0) {  // the whole cycle in one CTA: the dot products are a launch of their own
         cycle(0, z, rhs, nullptr);
@@ -562,11 +562,10 @@ int Poisson::vcycle(const float* rhs, float* z) {
         count = mg_sweep_ctas(lvdesc_[0]);
     }
     if (count > 2048) {  // every CTA of the next kernel sums the pairs: beyond 32 KB a launch of its own is cheaper
-        launch_finish(zpart_.d(), count, 2, 1.0, red_->res() + 8, s_);
-        KS_CUDA(cudaMemcpyAsync(zpart_.p, red_->res() + 8, 2 * sizeof(double), cudaMemcpyDeviceToDevice, s_));
-        count = 1;
+        launch_finish(zpart_.d(), count, 2, 1.0, scal_.d() + 5, s_);
+        return {scal_.d() + 5, 1};
     }
-    return count;
+    return {zpart_.d(), count};
 }
 
 // One PCG iteration between two readbacks (crates/qm-gpu/src/poisson.rs:284-342): ap = L p with p.Ap, the v / r update,
@@ -580,8 +579,8 @@ void Poisson::iteration(float* v, int par) {
     const int ctas = launch_stencil(L_, p_.tmap, 1, lapd, ap_.at(0), s_);
     // res[0] = p.Ap, res[1], res[2] = r.z, r.r: what the host reads after the iteration
     launch_cg_update(L_.F, v, r_.at(0), p_.at(0), ap_.at(0), red_->partials(), ctas, scal, 1 + 2 * par, red_->res(), s_);
-    const int count = vcycle(r_.at(0), z_.at(0));
-    launch_cg_direction(L_.F, p_.at(0), z_.at(0), zpart_.d(), count, scal, 1 + 2 * par, 1 + 2 * (1 - par), red_->res() + 1, s_);
+    const Pairs2 zr = vcycle(r_.at(0), z_.at(0));
+    launch_cg_direction(L_.F, p_.at(0), z_.at(0), zr.partials, zr.count, scal, 1 + 2 * par, 1 + 2 * (1 - par), red_->res() + 1, s_);
 }
 
 // The iteration's small launches (a few microseconds each) replayed as one CUDA
@@ -670,10 +669,10 @@ PoissonStats Poisson::solve(const float* rho, float* v, const CUtensorMap& v_map
     t.x[0] = b_.at(0); t.c[0] = 1.f;
     t.x[1] = ap_.at(0); t.c[1] = 1.f;
     launch_lincomb(L_.F, 1, r_.at(0), t, s_);
-    const int count = vcycle(r_.at(0), z_.at(0));
+    const Pairs2 zr = vcycle(r_.at(0), z_.at(0));
     red_->dots({{b_.at(0), b_.at(0)}}, 2, 1.0);
     // scal[1 + 2s] = r.z, scal[2 + 2s] = r.r for parity s
-    launch_cg_direction(L_.F, p_.at(0), z_.at(0), zpart_.d(), count, scal, -1, 1, red_->res(), s_);
+    launch_cg_direction(L_.F, p_.at(0), z_.at(0), zr.partials, zr.count, scal, -1, 1, red_->res(), s_);
     const double* h = red_->read(3);
     const double bb = h[2];
     double rz = h[0], rr = h[1];
@@ -792,6 +791,7 @@ size_t Solver::footprint_bytes(int n, int n_up, int n_dn, const SolverOptions& o
     total += 11 * rounded(field);                                        // potentials, densities, XC, ones
     total += 3 * (rounded(((size_t)1 << 20) * sizeof(double)) + rounded(Reducer::RES_CAP * sizeof(double)));  // reducers
     total += 6 * rounded(field) + rounded(24 * (size_t)n * n * sizeof(double));  // Poisson CG fields and ghost table
+    total += rounded(2 * (size_t)mg_sweep_ctas(MgLevel{n, L.P, L.F, 1.0, 0.f, 0.f}) * sizeof(double));  // the last sweep's dot partials
     for (int m = n; m > MG_COARSE_N;) {                                  // multigrid levels, three fields each
         m /= 2;
         total += 3 * rounded((size_t)Layout::make(m, 1.0).F * sizeof(float));

@@ -193,8 +193,9 @@ public:
 
 private:
     struct Level { MgLevel lv; DevBuf x, b, tmp; };
-    // z = M^-1 rhs by one V-cycle; leaves the partial pairs (rhs.z, rhs.rhs) in zpart_ and returns their count
-    int vcycle(const float* rhs, float* z);
+    // z = M^-1 rhs by one V-cycle; returns where the partial pairs (rhs.z, rhs.rhs) lie, and their count
+    struct Pairs2 { const double* partials; int count; };
+    Pairs2 vcycle(const float* rhs, float* z);
     void cycle(int l, float* x, const float* b, double* partials);
     void true_residual(const CUtensorMap& v_map);  // r = b + L v into ap_, |r|^2 reduced (v is v_map's field)
     void iteration(float* v, int par);

@@ -80,3 +80,24 @@ def test_vram_budget_refuses_before_building_a_solver():
         p.evaluate([(0.0, 0.0, 0.0, 8), (1.43, 1.11, 0.0, 1), (-1.43, 1.11, 0.0, 1)], 95, 0.25, 5, 5, ks.ScfSettings(sigma=0.5))
     assert p.solver is None
     p.check_vram(33, 5, 5, ks.ScfSettings(sigma=0.5))  # ~65 MiB fits
+
+
+@pytest.mark.parametrize("n", [129, 512, 1024])
+def test_footprint_counts_the_poisson_partials(n):
+    """What a one-spin solver without extra bands allocates on a large grid, buffer by buffer, among them one pair of f64
+    partials per CTA (32 x 8 columns of 4 points) of the Poisson solve's last sweep: 16 MiB at 1024^3."""
+    ks, _ = _drivers()
+
+    def rounded(b):
+        return (b + 2 ** 21 - 1) // 2 ** 21 * 2 ** 21 if b >= 2 ** 20 else (b + 511) // 512 * 512
+
+    def field(m):
+        return 4 * m * m * ((m + 3) // 4 * 4)
+    f, m, coarse = rounded(field(n)), n, 0
+    while m > 12:
+        m //= 2
+        coarse += 3 * rounded(field(m))
+    pairs = -(-n // 32) * -(-n // 8) * -(-n // 4)
+    want = 11 * f + 3 * (rounded(8 * 2 ** 20) + rounded(8 * 2 ** 16)) + 6 * f + rounded(24 * n * n * 8) + rounded(16 * pairs) + coarse
+    want += 3 * rounded(3 * field(n)) + 2 * f + rounded(8 * (2 + 6)) + 7 * 4 * f
+    assert ks.footprint_bytes(n, 1, 0, diis_history=6) == want
