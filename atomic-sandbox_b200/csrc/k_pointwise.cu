@@ -167,7 +167,7 @@ constexpr int LC_RING = 16;      // stages at most
 constexpr int LC_SETS = 3;
 constexpr int LC_THREADS = 960;  // consumer threads at most (with the producer warp 992: 64 registers each)
 constexpr int LC_SMEM = 216 * 1024;
-constexpr long long LC_WAIT_LIMIT = 1LL << 22;
+constexpr long long LC_WAIT_LIMIT = 1LL << 22, LC_DRAIN_LIMIT = 1LL << 16;
 __device__ __forceinline__ unsigned long long lc_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
@@ -208,7 +208,8 @@ __global__ void __launch_bounds__(LC_THREADS + 32, 1) block_lincomb_kernel(long 
     __syncthreads();
     if ((int)threadIdx.x >= consumers) {
         // ---- producer warp. A wait that gives up raises the error flag (the host's next readback reports it) and ends the
-        // loads; the copies in flight then get a bounded time to land before the CTA's shared memory is released.
+        // loads. The warp stays until its last copies have landed, for a bounded time that outlasts a consumer's own wait, so
+        // that no copy writes the CTA's shared memory after it is released, whichever wait gave up.
         const int lane = threadIdx.x & 31;
         int sl = 0, issued = 0;
         unsigned ph = 1;  // a fresh barrier passes a wait on the parity before its first phase
@@ -232,8 +233,9 @@ __global__ void __launch_bounds__(LC_THREADS + 32, 1) block_lincomb_kernel(long 
                              : "memory");
             if (++sl == sh.ring) { sl = 0; ph ^= 1u; }
         }
-        if (!__all_sync(0xffffffffu, alive))
-            for (int j = max(0, issued - sh.ring); j < issued; ++j) lc_wait(&full[j % sh.ring], (unsigned)((j / sh.ring) & 1), 1LL << 16);
+        const long long limit = __all_sync(0xffffffffu, alive) ? LC_WAIT_LIMIT + LC_DRAIN_LIMIT : LC_DRAIN_LIMIT;
+        for (int j = max(0, issued - sh.ring); j < issued; ++j)
+            if (!lc_wait(&full[j % sh.ring], (unsigned)((j / sh.ring) & 1), limit)) break;
         return;
     }
     // the coefficients while the first copies are in flight
