@@ -53,6 +53,7 @@ constexpr int THREADS = 480;                 // 8 epilogue, 4 split, 1 TMA, 2 MM
 constexpr int FLUSH = 8;                     // stages summed in f32 before an f64 add
 constexpr int NBUF_MAX = 8;                  // hi*hi accumulator buffers in flight (TMEM permitting)
 constexpr long long WAIT_LIMIT = 1LL << 24;
+constexpr int DRAIN_POLLS = 1 << 16;         // per copy in flight after a wait gave up
 
 __device__ __forceinline__ unsigned su32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -183,7 +184,11 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
             int s = 0;
             unsigned ph = 0;
             for (int i = 0; i < nst; ++i) {
-                if (i >= R && !mbar_wait(&empty[s], ph ^ 1u, p.err)) break;
+                if (i >= R && !mbar_wait(&empty[s], ph ^ 1u, p.err)) {
+                    for (int j = i - R; j < i; ++j)
+                        for (int polls = 0; polls < DRAIN_POLLS && !mbar_try(&full[j % R], (unsigned)((j / R) & 1)); ++polls) {}
+                    break;
+                }
                 mbar_expect_tx(&full[s], bytes);
                 unsigned char* dst = hi + (size_t)s * p.tbytes;
                 const int x = (s0 + i) * KT;
@@ -322,6 +327,12 @@ __global__ void __launch_bounds__(THREADS, 1) gram_tc_kernel(const __grid_consta
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // Whichever wait gave up, the last copies (lane t: the slot of the t-th last stage) get a bounded time to land before the
+    // CTA's shared memory is released; else all have, and this is one poll.
+    if (warp == 12 && lane < min(R, nst)) {
+        const int j = nst - 1 - lane;
+        for (int polls = 0; polls < DRAIN_POLLS && !mbar_try(&full[j % R], (unsigned)((j / R) & 1)); ++polls) {}
+    }
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
