@@ -170,8 +170,9 @@ def test_lobpcg_oscillator_matches_oracle(ks, oracle):
 
 @pytest.mark.parametrize("m,mt", [(8, 8), (24, 24), (10, 15), (60, 60)])
 def test_tensor_core_gram_matches_numpy(ks, m, mt):
-    """The 3xTF32 tcgen05 Gram (the "mixed" form): the same pairs as the CUDA-core Gram to ~1e-6
-    relative, including blocks whose row counts are not multiples of 8 and the largest block (60)."""
+    """The mixed form of the Gram: the same pairs as the plain form to ~1e-6 relative, including blocks whose row counts
+    are not multiples of 8 and the largest block (60), the one here that reaches the 3xTF32 tcgen05 kernel (blocks of at
+    most 32 columns take the CUDA cores; test_gpu_edges.py has the kernel's other shapes)."""
     n = 33 if m < 60 else 21
     rng = np.random.default_rng(m + mt)
     s = f32(rng.standard_normal((m, n ** 3)))
@@ -184,6 +185,7 @@ def test_tensor_core_gram_matches_numpy(ks, m, mt):
 
 
 def test_lobpcg_tensor_core_gram_matches_oracle(ks, oracle):
+    """The mixed form with 4 vectors: up to 12 columns, so the CUDA cores (the next test reaches the tensor cores)."""
     n, h = 33, 0.25
     x, y, z = oracle.grid_points(n, h)
     v = f32(0.5 * (x * x + y * y + z * z))
@@ -192,6 +194,23 @@ def test_lobpcg_tensor_core_gram_matches_oracle(ks, oracle):
     ev, xs, it, mr = ks.lobpcg(n, h, v, guess, tol=2e-5, max_iter=400, gram_mode=1)
     evo, _, _, _ = oracle.lobpcg(n, h, v, guess, tol=1e-8, max_iter=500, precond_lambda=1.5)
     assert np.abs(np.sort(ev) - np.sort(evo)).max() < 1e-5, (ev, evo)
+
+
+@pytest.mark.parametrize("k,w2", [(13, (1.0, 1.21, 1.69)), (20, (1.0, 1.0, 1.0))])
+def test_lobpcg_on_the_tensor_cores_matches_oracle(ks, oracle, k, w2):
+    """The mixed form where 3 k > 32 columns take the tensor-core Gram in every iteration with P: 39 columns (an
+    anisotropic oscillator with single levels) and 60 (four whole shells); the f64 eigenvalues on the same grid to 1e-5, as
+    with the plain form, and an orthonormal block."""
+    n, h = 25, 0.4
+    x, y, z = oracle.grid_points(n, h)
+    v = f32(0.5 * (w2[0] * x * x + w2[1] * y * y + w2[2] * z * z))
+    rng = np.random.default_rng(5)
+    guess = rng.uniform(-0.5, 0.5, (k, n ** 3)) * np.exp(-(x * x + y * y + z * z) / 8.0)
+    ev, xs, it, mr = ks.lobpcg(n, h, v, guess, tol=2e-5, max_iter=400, gram_mode=1)
+    evo, _, _, _ = oracle.lobpcg(n, h, v, guess, tol=1e-8, max_iter=500, precond_lambda=1.5)
+    assert np.abs(np.sort(ev) - np.sort(evo)).max() < 1e-5, (ev, evo)
+    gm = xs @ xs.T
+    assert np.abs(gm / np.sqrt(np.outer(gm.diagonal(), gm.diagonal())) - np.eye(k)).max() < 1e-5
 
 
 def _check_rel(name, got, want, mag, rel=1e-6):

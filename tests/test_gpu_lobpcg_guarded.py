@@ -56,8 +56,8 @@ def test_converged_block_is_accepted_at_the_guess(ks, rig):
 @pytest.mark.parametrize("gram_mode", [0, 1])
 def test_fresh_fifth_column_locks_the_head(ks, rig, gram_mode):
     """(b) the fifth column replaced by a fresh seed: the head is locked -- returned bitwise, head_kept -- and only the
-    fifth column iterates, to the guard tolerance, landing on 3.5 Ha, orthogonal to the head; with the CUDA-core and
-    the tensor-core Gram (the locked subspace [Y, X_a, W_a, P_a] has k + 2 (k - head) columns)."""
+    fifth column iterates, to the guard tolerance, landing on 3.5 Ha, orthogonal to the head; with the plain and the
+    mixed Gram (the locked subspace [Y, X_a, W_a, P_a] has k + 2 (k - head) columns: 7 here, the CUDA cores in both)."""
     v, xs, seed, tol = rig
     x0 = xs.copy()
     x0[4] = seed.astype(np.float32).astype(np.float64)
@@ -91,3 +91,26 @@ def test_untested_buffer_is_not_checked(ks, rig):
     ev, x, res, st = ks.lobpcg_guarded(N, H, v, x0, tol, 1.5 * tol, HEAD, GUARD, HEAD, max_iter=500, lock=False)
     assert st["iterations"] == 0 and st["head_kept"], st
     assert res[4] > GUARD  # measured, never tested
+
+
+def test_locked_block_on_the_tensor_cores(ks, oracle):
+    """(b) with a locked subspace of 20 + 2 * 10 = 40 columns, which the mixed form gives to the tensor cores: the first
+    three shells (10 columns, to 3.5 Ha) are locked and returned bitwise, the 4.5 Ha shell starts from fresh seeds and
+    reaches the guard tolerance, orthogonal to the head."""
+    n, h, k, head = 25, 0.4, 20, 10
+    x, y, z = oracle.grid_points(n, h)
+    r2 = x * x + y * y + z * z
+    v = (0.5 * r2).astype(np.float32).astype(np.float64)
+    rng = np.random.default_rng(12)
+    tol = 3.0 * floor_estimate(h)
+    _, x0, _, mr = ks.lobpcg(n, h, v, rng.uniform(-0.5, 0.5, (k, n ** 3)) * np.exp(-r2 / 8.0), tol=tol, max_iter=500, gram_mode=1)
+    assert mr <= tol, mr
+    x0[head:] = (rng.uniform(-0.5, 0.5, (k - head, n ** 3)) * np.exp(-r2 / 8.0)).astype(np.float32).astype(np.float64)
+    ev, xs, res, st = ks.lobpcg_guarded(n, h, v, x0, tol, 1.5 * tol, head, GUARD, k, max_iter=500, gram_mode=1)
+    assert st["iterations"] > 1 and st["head_kept"] and st["locked"] == head, st
+    assert np.array_equal(xs[:head], x0[:head]), "the locked head is returned bitwise"
+    # a residual below the guard bounds the level to GUARD, the grid's own levels lie within 6e-4 of 4.5
+    assert (res[head:] < GUARD).all() and np.abs(ev[head:] - 4.5).max() < 2.0 * GUARD, (ev, res)
+    gm = xs @ xs.T
+    cos = np.abs(gm / np.sqrt(np.outer(gm.diagonal(), gm.diagonal())) - np.eye(k)).max()
+    assert cos < 1e-5, cos

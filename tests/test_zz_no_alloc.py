@@ -59,3 +59,34 @@ def test_noalloc_gram_rejects_a_block_beyond_its_scratch(ks):
         ks.gram_device_noalloc(torch.cuda.current_stream().cuda_stream, n, m, S.data_ptr(), mt, S[m:].data_ptr(),
                                out.data_ptr())
     assert ks.launch_count() == before
+
+
+def test_noalloc_gram_of_4_byte_aligned_fields(ks):
+    """Fields on 4-byte boundaries: blocks of more than 16 tiles of 8 x 8 take the direct form, which reads single floats;
+    smaller ones are refused, as before. Against the f64 products to the Gram tests' 2e-6."""
+    import torch
+
+    n, m, mt = 9, 8, 128  # 1 + 16 tiles
+    P = ks.field_pitch(n)
+    rng = np.random.default_rng(3)
+    s, t = rng.standard_normal((m, n ** 3)), rng.standard_normal((mt, n ** 3))
+
+    def shifted(dense):
+        block = _device_fields(torch, ks, n, dense)
+        flat = torch.zeros(block.numel() + 4, dtype=torch.float32, device="cuda:0")
+        flat[1:-3] = block.flatten()
+        return flat[1:]
+    S, T = shifted(s), shifted(t)
+    assert S.data_ptr() % 16 == 4
+    stream = torch.cuda.current_stream().cuda_stream
+    out = torch.full((m, m + mt), float("nan"), dtype=torch.float64, device="cuda:0")
+    ks.gram_device_noalloc(stream, n, m, S.data_ptr(), mt, T.data_ptr(), out.data_ptr())
+    torch.cuda.synchronize()
+    s32, t32 = s.astype(np.float32).astype(np.float64), t.astype(np.float32).astype(np.float64)
+    cols = np.concatenate([s32, t32])
+    scale = np.sqrt(np.outer((s32 * s32).sum(1), (cols * cols).sum(1)))
+    assert (np.abs(out.cpu().numpy() - s32 @ cols.T) / scale).max() < 2e-6
+    before = ks.launch_count()
+    with pytest.raises(ValueError, match="16-byte aligned"):
+        ks.gram_device_noalloc(stream, n, m, S.data_ptr(), 8, T.data_ptr(), out.data_ptr())
+    assert ks.launch_count() == before
