@@ -1000,8 +1000,8 @@ ks_status ks_device_status(void* stream) {
 ks_status ks_gram_device_noalloc(void* stream, int n, int m, const float* s, int mt, const float* t, double* out) {
     if (n < 5 || n > 1024 || m < 1 || mt < 0 || !s || (mt > 0 && !t) || !out) return fail(nullptr, KS_INVALID, "invalid arguments");
     return guarded(nullptr, [&] {
-        // the solver's CUDA-core Gram kernel and grid, hence the same partials and result; it writes at most 2 * SMs
-        // partial blocks, the bound the scratch is sized against
+        // the solver's CUDA-core Gram kernel and grid, hence the same partials and result. It writes at most one partial
+        // block per SM (gram_blocks); the published limit stays at two, so that what is refused does not depend on the grid
         const int blocks = 2 * sm_count();
         const size_t need = (size_t)blocks * m * (m + mt);
         if (need > NOALLOC_PARTIALS)

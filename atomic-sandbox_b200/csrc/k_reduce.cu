@@ -173,9 +173,10 @@ __global__ void __launch_bounds__(GW * 32) gram_kernel(long long F, int m, const
 // redundant are skipped, and with LOWER also those of S^T T above the diagonal, which a Rayleigh-Ritz step never reads
 // (24 patches instead of 30).
 // Measured (with the finish): m = mt = 24 on 95^3 99.7 -> 57.3 us, 8 / 8 69 -> 24.6, 128^3 24 / 24 208 -> 114, 48^3 12 / 12 25.8 ->
-// 16.4; in a solve, where LOWER applies, 96.7 -> 49.6 us. At 3.3 TB/s it is bound by the FMA pipe
-// (58 % active, math_pipe_throttle first) and fixed latencies at 12 to 16 warps per SM. Scalar FMAs took the same time. Rows of 512 bytes by one bulk
-// copy each, at a padded pitch, measured slower: 85 us copied by the consumers, 95 us by a producer warp.
+// 16.4; in a solve, where LOWER applies, 96.7 -> 49.6 us. At 3.3 TB/s no unit is above 60 %: three or four warps per scheduler
+// leave the FMA pipe (58 % active) throttled while they multiply in bursts and idle while the operands load. Scalar FMAs took the
+// same time. Rows of 512 bytes by one bulk copy each, at a padded pitch, measured slower: 85 us copied by the consumers, 95 us
+// by a producer warp.
 // Sums: f32 over 16 points of a slab, f32 over a warp's slabs, f64 across the warps and (launch_finish) the CTAs.
 // Larger blocks are several pieces: DIAG pieces (rows, the same columns of S and of T) and pieces of one foreign column block.
 constexpr int GP = 32;             // points per slab (one 128-byte swizzle row)
@@ -320,7 +321,9 @@ __global__ void __launch_bounds__(32 * g_warps<M8, T8, DIAG, LOWER>(), 1)
     if (!alive && lane == 0)
         for (int k = max(0, issued - DEPTH); k < issued; ++k) g_wait(&bars[k % DEPTH], (unsigned)((k / DEPTH) & 1), 1LL << 16);
     __syncthreads();
-    // across the warps in f64, from the last warp to the first (the last ones hold the fewest slabs)
+    // across the warps in f64, from the last warp to the first. Either direction is as exact; the direction was chosen because
+    // solves that end at the f32 residual floor are sensitive to the last bit of these sums, and with it all of the tests'
+    // tight warm solves converge in the steps that they allow.
     float* red = reinterpret_cast<float*>(base);  // [warp][patch][lane]
 #pragma unroll
     for (int i = 0; i < RI; ++i)

@@ -12,16 +12,17 @@
 // map's extent is n on every axis, so the halo beyond the box arrives as the hardware's zero fill -- the Dirichlet
 // boundary costs no branches and no ghost storage. A ring of 8 planes keeps up to four planes of prefetch in flight.
 // Each thread owns four consecutive x-outputs of two adjacent rows: it reads its centre, x- and y-neighbours as 16-byte
-// quads (13 shared loads per 8 outputs, the ten y-rows serving both output rows) and works on packed pairs with
-// Blackwell's f32x2 arithmetic. The z-direction holds no queue of planes: a new plane's second difference is added to the
-// seven outputs it belongs to (ZRow), so nothing moves between registers. The V / R reads (cp.async copies one plane ahead
-// into a small shared ring) and the stores are coalesced 16-byte accesses; the quad's pad columns are stored as 0.
+// quads (16 shared loads per 8 outputs: the new plane's two, the centre's two, four x-neighbours and eight more y-rows, ten
+// rows serving both output rows) and works on packed pairs with Blackwell's f32x2 arithmetic. The z-direction holds no queue
+// of planes: a new plane's second difference is added to the seven outputs it belongs to (ZRow), so nothing moves between
+// registers. The V / R reads (cp.async copies one plane ahead into a small shared ring) and the stores are coalesced 16-byte
+// accesses; the quad's pad columns are stored as 0.
 //
 // What bounds it: instruction issue and the fixed latencies behind it at 12 warps per SM (58 % of the issue slots, FMA pipe
 // 53 % active). With one row per thread, a nine-deep register queue in z and symmetric differences (the form this
-// replaces) 128 outputs took 250 warp instructions, now 173. Measured per launch, before and after: H psi on 95^3 x 16
-// vectors 43.0 -> 34.9 us, on 128^3 x 40 216 -> 170 us, on 48^3 x 8 8.3 -> 7.2 us, a sweep on 128^3 x 20 in a solve
-// 160 -> 125 us.
+// replaces) 128 outputs took 250 warp instructions, now 173. Measured per launch, before and after, H psi back to back: 95^3 x
+// 16 vectors 43.0 -> 34.9 us, 128^3 x 40 216 -> 170 us, 48^3 x 8 8.3 -> 7.2 us, 33^3 x 3 5.4 -> 4.9 us of device time; a sweep on
+// 128^3 x 20 in a solve 160 -> 125 us.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -39,8 +40,9 @@ typedef unsigned long long u64;
 constexpr int BY = 16;                              // tile rows
 constexpr int HYW = BY + 8;
 constexpr int ROWS = 2;                             // adjacent rows per thread
-// A tile of BX columns: the staged plane with its halo, and one thread per x-quad and row pair. 12 warps per SM in every
-// width (registers capped at 168 per thread): 6 CTAs of 64 threads, 4 of 96 or 3 of 128.
+// A tile of BX columns: the staged plane with its halo, and one thread per x-quad and row pair. 12 warps per SM (registers
+// capped at 168 per thread): 6 CTAs of 64 threads, 4 of 96 or 3 of 128; only the sweep at BX = 32 holds 10, since the shared
+// memory of its larger side ring (39 KB per CTA) fits 5 times.
 template <int BX>
 struct Tile {
     static constexpr int HXW = BX + 8;
@@ -64,8 +66,8 @@ struct Tile {
 template <int MODE>
 constexpr int ring_depth() { return MODE == ST_JACOBI ? 7 : 8; }
 // The per-plane global reads of a step (V; r and the stored factor in the Jacobi mode) are staged one plane ahead by
-// per-thread cp.async copies into a 2-deep shared "side" ring (12 KB per CTA in the Jacobi mode, 4 KB for H and the
-// residual form), so their latency runs behind the previous plane's arithmetic without holding registers.
+// per-thread cp.async copies into a 2-deep shared "side" ring (at BX = 32, 48, 64: 12, 18, 24 KB per CTA in the Jacobi mode, 4,
+// 6, 8 KB for H and the residual form), so their latency runs behind the previous plane's arithmetic without holding registers.
 constexpr int SD = 2;
 template <int MODE>
 constexpr int n_side() { return MODE == ST_JACOBI ? 3 : (MODE == ST_LAPLACIAN ? 0 : 1); }
@@ -150,7 +152,9 @@ __device__ __forceinline__ void tma_load_plane(float* dst, const CUtensorMap* ma
 }
 
 // Before a TMA load refills a ring slot: the barrier orders the CTA's reads of the slot before this thread, the fence
-// orders them before the load's writes, which are the async proxy's. Without it reads that were still in flight when
+// orders them before the load's writes, which are the async proxy's. What counts is one proxy fence on the path from the
+// reads to the load: here the barrier makes the issuing thread's enough; where the readers signal an mbarrier instead (the
+// block update, the CUDA-core Gram) they fence before they signal. Without it reads that were still in flight when
 // the barrier released thread 0 could see the new plane: with kernels of three streams on the chip, solves stopped
 // being bit for bit reproducible.
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -483,9 +487,9 @@ struct Shape { int tiles_x, tiles_y, chunks, zc; };
 
 // The tile width of an n^3 grid: the fewest tile columns for the work in them. A tile's plane costs its arithmetic, which
 // grows with the width, but no less than a fixed part (the 24 TMA rows, the barrier), about that of 42 columns: a row of tiles
-// costs tiles x max(264, 6.25 BX). Measured per launch with every width forced to 32 / 48 / 64 (us): the sweep at 48^3 k = 4
-// 10.9 / 10.7 / 10.7 and H at k = 8 12.9 / 10.7 / 12.7; 64^3 k = 8 16.2 / 18.9 / 14.8; 95^3 k = 8 31.2 / 29.1 / 36.7; 128^3
-// k = 20 147 / 158 / 125; H at 128^3 k = 40 177 / 197 / 176.
+// costs tiles x max(264, 6.25 BX). Measured with every width forced to 32 / 48 / 64 (us, events around each launch of a solve,
+// which add up to 5 us to the shortest): the sweep at 48^3 k = 4 10.9 / 10.7 / 10.7 and H at k = 8 12.9 / 10.7 / 12.7; 64^3 k = 8
+// 16.2 / 18.9 / 14.8; 95^3 k = 8 31.2 / 29.1 / 36.7; 128^3 k = 20 147 / 158 / 125; H at 128^3 k = 40 177 / 197 / 176.
 int tile_width(int n) {
     int best = 32;
     double cost = 1e30;
@@ -517,7 +521,8 @@ int ctas_per_sm(int mode, int bx) {
 // whatever else runs, and the launch takes ceil(CTAs / resident slots) such rounds, so the chunk count minimises
 // waves x (zc + c) with c the fixed cost of a chunk in plane steps (its 8 halo planes, partly hidden behind the other
 // resident CTAs; c = 8 measured best against 12 and 4). Chunks go down to 4 planes, which only grids that leave the chip
-// idle reach (33^3 x 3: 6.2 us against 8.3 us with chunks of 8).
+// idle reach. Device time of a call there: 33^3 x 3 with 7 chunks of 5 planes 4.9 us, with 4 of 9 6.8 us; 48^3 x 4 with 12 of
+// 4 planes 4.5 us, with 6 of 8 6.3 us.
 Shape shape_for(const Layout& L, int count, int mode) {
     const int bx = tile_width(L.n);
     Shape sh;

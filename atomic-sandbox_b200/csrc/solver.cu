@@ -368,7 +368,6 @@ void Reducer::init(const Layout& L, cudaStream_t s, size_t partial_doubles) {
     L_ = L;
     s_ = s;
     blocks_ = reduce_blocks(L.F);
-    gram_blocks_ = 2 * sm_count();
     partials_.alloc(std::max(partial_doubles, (size_t)1 << 16) * sizeof(double));
     res_.alloc(RES_CAP * sizeof(double));
     KS_CUDA(cudaMallocHost(&host_, RES_CAP * sizeof(double)));

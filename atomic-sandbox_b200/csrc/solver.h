@@ -118,7 +118,6 @@ private:
     double* host_ = nullptr;
     int* host_flag_ = nullptr;
     int blocks_ = 1;
-    int gram_blocks_ = 1;
 
 public:
     ~Reducer();

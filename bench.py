@@ -13,8 +13,9 @@ a barrier + synchronize on both sides of the timed region; the max over ranks. `
 time of the user-facing calls (ks_solve + ks_forces + ks_state_density: nuclei in from host memory,
 energy, forces and both spin densities out to host memory, the densities into page-locked buffers allocated once).
 
-Forms: "plain FP32" = the LOBPCG Gram on CUDA cores, "mixed" = the Gram on the tensor cores
-(3xTF32); FP64 stays in the Rayleigh-Ritz, DIIS and every reduction finish in both.
+Forms: "plain FP32" = the LOBPCG Gram on CUDA cores, "mixed" = the Gram on the tensor cores (3xTF32) for blocks of more
+than 32 columns; this workload's 24 columns take the CUDA cores in both. FP64 stays in the Rayleigh-Ritz, DIIS and
+every reduction finish in both.
 
 --impl reference times the reference's CPU algorithm (the f64 C++ restatement under oracle/, all
 host threads) solving the whole workload once (a measured full SCF + forces, minutes of CPU); rank 0 only.
@@ -413,8 +414,9 @@ def bench_ours(args):
 
 def kernel_only(args):
     """One hot kernel in isolation, for profiling: --kernel hpsi (H psi on a --count block of 95^3
-    fields, timed as in the roofline) or --kernel gram (the LOBPCG Gram G = S^T [S | T] at 95^3 with
-    m = mt = 24, through ks_gram; --form plain runs the CUDA-core form)."""
+    fields, timed as in the roofline) or --kernel gram (the LOBPCG Gram G = S^T [S | T] at 95^3 through
+    ks_gram: m = mt = 60, which the mixed form gives to the tensor cores, or with --form plain
+    m = mt = 24 on the CUDA cores)."""
     import torch
     import ks_b200 as ks
     peak, source = measured_peaks()
@@ -423,12 +425,13 @@ def kernel_only(args):
         return
     import numpy as np
     rng = np.random.default_rng(5)
-    s = rng.standard_normal((24, N ** 3))
-    t = rng.standard_normal((24, N ** 3))
     gm = 0 if args.form == "plain" else 1
+    m = 60 if gm else 24
+    s = rng.standard_normal((m, N ** 3))
+    t = rng.standard_normal((m, N ** 3))
     for _ in range(4):
         g = ks.gram(N, s, t, gram_mode=gm)
-    print(json.dumps({"kernel": "gram", "gram_mode": gm, "n": N, "m": 24, "mt": 24, "g00": float(g[0, 0])}), flush=True)
+    print(json.dumps({"kernel": "gram", "gram_mode": gm, "n": N, "m": m, "mt": m, "g00": float(g[0, 0])}), flush=True)
 
 
 def bench_batch(args):

@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 REC = json.load(open(os.path.join(os.path.dirname(__file__), "golden", "oracle_h3plus_49.json")))
 
 
-@pytest.mark.parametrize("gram_mode", [0, 1])  # the plain and the mixed (tensor-core Gram) form
+@pytest.mark.parametrize("gram_mode", [0, 1])  # the plain and the mixed form
 def test_stretched_h3plus_converges_cold(ks, gram_mode):
     nuc = [tuple(a) for a in REC["nuclei"]]
     settings = ks.ScfSettings.for_grid(REC["h"])
