@@ -106,9 +106,9 @@ def test_poisson_level_edges(ks, oracle, n):
                                     (21, 48, 48), (13, 49, 1), (13, 49, 72), (21, 56, 56), (21, 57, 57), (13, 64, 64)])
 def test_tensor_core_gram_shapes(ks, n, m, mt):
     """Every class of N = round16(m) of the tensor-core form against round8(m), with T blocks up to the largest, one stage
-    per CTA and several. Bound: hi holds 11 bits, so the dropped lo lo term is below 2^-20 |s| |t|, the two rounded lo
-    operands add 2^-22 each, and the truncating sums of a stage's 12 products at most 12 ulp of 2^-24 between them:
-    together under 2e-6."""
+    per CTA and several. Bound: hi holds 11 bits, so the dropped lo lo term is below 2^-20 |s| |t|, over uniform mantissas
+    a sixth of that in the mean; the two rounded lo operands add 2^-22 each, the truncating sums of a stage's 12 products at
+    most 12 times 2^-24: 1.4e-6 together, under the 2e-6 of the other tests."""
     rng = np.random.default_rng(100 * m + mt)
     s, t = f32(rng.standard_normal((m, n ** 3))), f32(rng.standard_normal((mt, n ** 3)))
     g = ks.gram(n, s, t, gram_mode=1)
